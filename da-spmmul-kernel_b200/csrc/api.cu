@@ -354,13 +354,29 @@ static daspmm_status dispatch(const Resolved &r, KArgs &a, dim3 grid, dim3 fix_g
 }
 
 // dst (Cn x R, row-major) = transpose of src (R x Cn, row-major) + beta * dst.
+template <int TR>
+static void launch_transpose_tr(const float *src, long long R, long long Cn, float *dst,
+                                float beta, cudaStream_t st)
+{
+    constexpr int TC = 4096 / TR;
+    const long long tiles = ((R + TR - 1) / TR) * ((Cn + TC - 1) / TC);
+    const unsigned g = (unsigned)std::max<long long>(
+        1, std::min<long long>(tiles, (long long)device_sms() * 8));
+    const bool vl = Cn % 4 == 0 && aligned(src, 16), vs = R % 4 == 0 && aligned(dst, 16);
+    if (vl && vs) k_transpose<TR, true, true><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
+    else if (vl) k_transpose<TR, true, false><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
+    else if (vs) k_transpose<TR, false, true><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
+    else k_transpose<TR, false, false><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
+}
+
 static void launch_transpose(const float *src, long long R, long long Cn, float *dst, float beta,
                              cudaStream_t st)
 {
-    const long long tiles = ((R + 31) / 32) * ((Cn + 31) / 32);
-    const unsigned g = (unsigned)std::max<long long>(
-        1, std::min<long long>(tiles, (long long)device_sms() * 16));
-    k_transpose<<<g, dim3(32, 8), 0, st>>>(src, R, Cn, dst, beta);
+    if (R <= 16) launch_transpose_tr<16>(src, R, Cn, dst, beta, st);
+    else if (R <= 32) launch_transpose_tr<32>(src, R, Cn, dst, beta, st);
+    else if (Cn <= 16) launch_transpose_tr<256>(src, R, Cn, dst, beta, st);
+    else if (Cn <= 32) launch_transpose_tr<128>(src, R, Cn, dst, beta, st);
+    else launch_transpose_tr<64>(src, R, Cn, dst, beta, st);
     count_launches(1);
 }
 
