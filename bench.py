@@ -434,7 +434,7 @@ def run_ours(args):
             "variant": dict(cfg_used.as_dict(), alg_name=alg.name),
             "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                          "unit": "GB/s", "frac": round(achieved / peak, 4),
-                         "traffic": traffic, "kernel": "k_bal_grp<16,8,8,float,float> (the main gather; CUDA events around each "
+                         "traffic": traffic, "kernel": "k_win<16,8,1,8,float,float> (the main gather; CUDA events around each "
                                    "launch of it in a second pass of K calls)",
                          "kernel_ms": round(kern_ms, 5), "algorithmic_bytes": abytes,
                          "gather_upper_bound_bytes": gather_bytes(A, NV),
@@ -459,8 +459,8 @@ def run_ours(args):
 
 def run_plan(D, A, dA, Bt, dev, peak, K):
     """The same product through a plan (daspmm_plan_*): the balanced split's
-    boundaries computed once, each step one window-kernel launch (plus the
-    walk over listed chunks, none on this matrix).  K steps back to back
+    boundaries computed once, each step one window-kernel launch (this matrix
+    has no row without nonzeros).  K steps back to back
     between CUDA events, after 5 warm-up steps; the result is compared bit for
     bit with the stateless call's."""
     import torch
@@ -496,7 +496,7 @@ def run_plan(D, A, dA, Bt, dev, peak, K):
             "kernel_frac": round(abytes / (kms * 1e-3) / 1e9 / peak, 4),
             "bit_identical_to_stateless": same,
             "what": "daspmm_plan_spmm: boundaries computed once at plan creation; per step the "
-                    "window kernel and the walk over listed chunks"}
+                    "window kernel"}
 
 
 REF_VARIANTS = [  # run.sh:29 column order: alg (spmvspmm.h:5-10) x layout

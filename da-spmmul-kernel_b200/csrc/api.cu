@@ -10,7 +10,7 @@
 #include "daspmm.h"
 #include "kernels.cuh"
 #include "gather_tma.cuh"
-#include "gather_lean.cuh"
+#include "gather_win.cuh"
 #include "internal.h"
 
 #include <cuda_runtime.h>
@@ -92,6 +92,27 @@ static int pow2ceil(int x)
 static bool is_pow2(int x) { return x > 0 && (x & (x - 1)) == 0; }
 static bool aligned(const void *p, size_t a) { return ((uintptr_t)p % a) == 0; }
 
+// The widest of 4, 2 and 1 floats that row-major rows of nv floats at B and C
+// can be accessed by.
+static int default_vec(int nv, const void *B, const void *C)
+{
+    if (nv % 4 == 0 && (!B || aligned(B, 16)) && (!C || aligned(C, 16))) return 4;
+    if (nv % 2 == 0 && (!B || aligned(B, 8)) && (!C || aligned(C, 8))) return 2;
+    return 1;
+}
+
+// Tile width of the masked window kernel for nv columns in vectors of V: as few
+// tiles of at most 128 columns as cover nv, each the narrowest width that does
+// (a lane past nv is idle, so 132 columns take two tiles of 96, not of 128).
+static int general_width(int V, int nv)
+{
+    const int n = (nv + 127) / 128, per = (nv + n - 1) / n;
+    if (per <= 32) return 32;
+    if (per <= 48 && V == 1) return 48;
+    if (per <= 64) return 64;
+    return per <= 96 ? 96 : 128;
+}
+
 // ---------------------------------------------------------------- resolve
 daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int nnz, int nv,
                       const void *B, const void *C, Resolved *out)
@@ -142,9 +163,7 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
         if (C && !aligned(C, 4 * cfg->vec)) return DASPMM_ERR_INVALID;
         r.V = cfg->vec;
     } else {
-        r.V = 1;
-        if (nv % 4 == 0 && (!B || aligned(B, 16)) && (!C || aligned(C, 16))) r.V = 4;
-        else if (nv % 2 == 0 && (!B || aligned(B, 8)) && (!C || aligned(C, 8))) r.V = 2;
+        r.V = default_vec(nv, B, C);
     }
     const int vecs = (nv + r.V - 1) / r.V;  // vectors across a dense row
     // coarsening factor
@@ -171,12 +190,17 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
     if ((cfg->alg == DASPMM_ALG_COO_SCALAR || cfg->alg == DASPMM_ALG_CSR_BALANCED) && r.S != 1)
         return DASPMM_ERR_UNSUPPORTED;
     const int G = r.L * r.S;
+    // every field of the shape is zero or what zero would give
+    daspmm_config d = *cfg;
+    const bool plain_shape = (!d.vec || d.vec == default_vec(nv, B, C)) &&
+                             (!d.cf || d.cf == (vecs > 32 ? 2 : 1)) &&
+                             (!d.lanes_col || d.lanes_col == std::min(32, pow2ceil((vecs + r.CF - 1) / r.CF)));
     // chunks
     if (cfg->alg >= DASPMM_ALG_COO_SCALAR) {
         if (cfg->chunk) r.chunk = cfg->chunk;
         else if (cfg->alg == DASPMM_ALG_COO_VECTOR) r.chunk = std::max(64, 8 * r.S);
         else if (r.cm) r.chunk = 32;
-        else r.chunk = G >= 32 ? 128 : (G >= 16 ? 64 : 32);
+        else r.chunk = G >= 32 ? 128 : (G >= 16 || (!r.cm && nv > 16) ? 64 : 32);
         if (r.chunk < 1) return DASPMM_ERR_INVALID;
         if (cfg->alg == DASPMM_ALG_COO_VECTOR && r.chunk % r.S) return DASPMM_ERR_INVALID;
         r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
@@ -223,11 +247,23 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
             }
         }
     }
-    const int W = r.L * r.V * r.CF;
+    if (r.pipe == 1 && cfg->alg == DASPMM_ALG_CSR_BALANCED && !r.cm && nv > 16 && plain_shape) {
+        // the shape is the library's: the window kernel with masked columns
+        r.general = r.V;
+        r.W = general_width(r.V, nv);
+        r.block = 256;
+    }
+    const int W = r.general ? r.W : r.L * r.V * r.CF;
     r.tiles = (nv + W - 1) / W;
     if (r.tiles > 65535) return DASPMM_ERR_UNSUPPORTED;
     *out = r;
     return DASPMM_OK;
+}
+
+// Does the window kernel run this product (after k_partition, no fix-up)?
+static bool windowed(const Resolved &r)
+{
+    return r.alg == DASPMM_ALG_CSR_BALANCED && (r.pipe == 4 || r.general);
 }
 
 // The row-major product inside pipe 5.
@@ -240,7 +276,16 @@ static daspmm_status resolve_inner(const Resolved &r, int nv, const void *B, con
     return resolve(&c, DASPMM_ROW_MAJOR, r.nr, r.nc, r.nnz, nv, B, C, in);
 }
 
-size_t workspace_bytes(const Resolved &r, int nv)
+// The window kernel's bitmap of empty rows, at the end of the workspace; a
+// workspace without room for it is still enough.
+static size_t emap_bytes(const Resolved &r)
+{
+    return windowed(r) ? align256(((size_t)r.nr + 31) / 32 * sizeof(unsigned int)) : 0;
+}
+
+size_t workspace_bytes(const Resolved &r, int nv) { return workspace_least(r, nv) + emap_bytes(r); }
+
+size_t workspace_least(const Resolved &r, int nv)
 {
     if (r.pipe == 5) {  // [B row-major | C row-major | the row-major product's own]
         Resolved in;
@@ -252,8 +297,7 @@ size_t workspace_bytes(const Resolved &r, int nv)
     if (r.alg == DASPMM_ALG_CSR_BALANCED) {
         b += align256(sizeof(int2) * ((size_t)r.nchunks + 1));
         b += align256(sizeof(int) * (size_t)r.nchunks * r.tiles);  // split-row arrival counters
-        b += align256(sizeof(unsigned int) * (size_t)r.tiles);     // chunk queue heads
-        b += align256(sizeof(int) * ((size_t)r.nchunks + 1));      // chunks left to the walk
+        b += align256(sizeof(unsigned int) * (size_t)r.tiles);  // chunk queue heads
     }
     if (r.alg >= DASPMM_ALG_COO_SCALAR) b += align256(sizeof(float) * 2 * (size_t)r.nchunks * nv);
     return b;
@@ -283,18 +327,38 @@ static void launch_ring(const Resolved &r, const KArgs &a, cudaStream_t st)
     else launch_tma_w<32, 4, MODE>(r, a, st);
 }
 
-template <int W>
-static void launch_lean_w(const Resolved &r, const KArgs &a, cudaStream_t st)
+// The window kernel over any width and alignment (the vector of `general`
+// floats divides both): the tile widths of general_width, columns past nv masked.
+static void launch_general(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
-    launch_lean<W, float, float, false>(r, a, st);
+    using F = float;
+    if (r.general == 4) {
+        if (r.W == 32) launch_win_as<8, 4, 1, 8, F, F, 3, true>(r, a, st);
+        else if (r.W == 64) launch_win_as<16, 4, 1, 8, F, F, 3, true>(r, a, st);
+        else if (r.W == 96) launch_win_as<8, 4, 3, 4, F, F, 2, true>(r, a, st);
+        else launch_win_as<16, 4, 2, 8, F, F, 2, true>(r, a, st);
+    } else if (r.general == 2) {
+        if (r.W == 32) launch_win_as<16, 2, 1, 16, F, F, 3, true>(r, a, st);
+        else if (r.W == 64) launch_win_as<16, 2, 2, 8, F, F, 3, true>(r, a, st);
+        else if (r.W == 96) launch_win_as<16, 2, 3, 8, F, F, 2, true>(r, a, st);
+        else launch_win_as<16, 2, 4, 8, F, F, 2, true>(r, a, st);
+    } else {
+        if (r.W == 32) launch_win_as<16, 1, 2, 16, F, F, 3, true>(r, a, st);
+        else if (r.W == 48) launch_win_as<16, 1, 3, 8, F, F, 3, true>(r, a, st);
+        else if (r.W == 64) launch_win_as<16, 1, 4, 8, F, F, 3, true>(r, a, st);
+        else if (r.W == 96) launch_win_as<16, 1, 6, 8, F, F, 2, true>(r, a, st);
+        else launch_win_as<16, 1, 8, 8, F, F, 2, true>(r, a, st);
+    }
 }
 
 static void launch_tma(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
-    if (r.pipe == 4) {
-        if (r.W == 128) launch_lean_w<128>(r, a, st);
-        else if (r.W == 64) launch_lean_w<64>(r, a, st);
-        else launch_lean_w<32>(r, a, st);
+    if (r.general) {
+        launch_general(r, a, st);
+    } else if (r.pipe == 4) {
+        if (r.W == 128) launch_lean<128, float, float, false>(r, a, st);
+        else if (r.W == 64) launch_lean<64, float, float, false>(r, a, st);
+        else launch_lean<32, float, float, false>(r, a, st);
     } else if (r.pipe == 3) {
         launch_ring<1>(r, a, st);
     } else {
@@ -322,13 +386,13 @@ static void launch_all(const Resolved &r, KArgs &a, dim3 grid, dim3 fix_grid, in
         k_eb_coo_pr<CM, V, CF><<<grid, block, 0, st>>>(a);
         break;
     case DASPMM_ALG_CSR_BALANCED:
-        if (r.pipe >= 2) launch_tma(r, a, st);
+        if (r.pipe >= 2 || r.general) launch_tma(r, a, st);
         else k_bal<CM, V, CF, false><<<grid, block, 0, st>>>(a);
         break;
     }
     timer_after(st);
     count_launches(1);
-    if (fix && r.alg >= DASPMM_ALG_COO_SCALAR && !(r.alg == DASPMM_ALG_CSR_BALANCED && r.pipe == 4)) {
+    if (fix && r.alg >= DASPMM_ALG_COO_SCALAR && !windowed(r)) {
         if (r.alg == DASPMM_ALG_CSR_BALANCED) k_fix_bal<CM, V, CF><<<fix_grid, block, 0, st>>>(a);
         else k_fix_coo<CM, V, CF><<<fix_grid, block, 0, st>>>(a);
         count_launches(1);
@@ -401,7 +465,7 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
     if (nnz > 0 && (!colIdx || !values)) return DASPMM_ERR_INVALID;
     if (coo ? (nnz > 0 && !rowIdx) : !rowPtr) return DASPMM_ERR_INVALID;
     if (nc <= 0 && nnz > 0) return DASPMM_ERR_INVALID;
-    const size_t need = workspace_bytes(r, nv);
+    const size_t need = workspace_least(r, nv);
     if (need > ws_bytes || (need && !ws)) return DASPMM_ERR_WORKSPACE;
 
     if (r.pipe == 5) {
@@ -446,8 +510,8 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
         }
         a.slots = (float *)ws;
     } else if (r.alg == DASPMM_ALG_CSR_BALANCED) {
-        carve_balanced(r, ws, &a);
-        launch_partition(r, nr, nnz, rowPtr, a, st);
+        carve_balanced(r, ws, ws_bytes, &a);
+        launch_partition(r, nr, nnz, rowPtr, a, windowed(r), st);
     }
     const long long units =
         (r.alg == DASPMM_ALG_CSR_SCALAR || r.alg == DASPMM_ALG_CSR_VECTOR) ? nr : r.nchunks;
@@ -461,12 +525,9 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
 
 bool run_planned(const Resolved &r, int nr, int nc, int nnz, int nv, const int *rowPtr,
                  const int *colIdx, const float *values, const float *B, float *C, void *ws,
-                 unsigned long long call, cudaStream_t st)
+                 size_t ws_bytes, const int *empty, int nempty, unsigned long long call, cudaStream_t st)
 {
     if (r.alg != DASPMM_ALG_CSR_BALANCED || r.cm || r.pipe != 4 || nr <= 0) return false;
-    // chunks per group of the window kernel: 32 / (W / 8) workers per warp
-    const int nw = r.W == 128 ? 2 : 4;
-    const unsigned long long ngroups = ((unsigned long long)r.nchunks + nw - 1) / nw;
     KArgs a{};
     a.nr = nr; a.nc = nc; a.nnz = nnz; a.nv = nv;
     a.ldb = nv; a.ldc = nv;
@@ -475,37 +536,44 @@ bool run_planned(const Resolved &r, int nr, int nc, int nnz, int nv, const int *
     a.L = r.L; a.S = r.S; a.chunk = r.chunk; a.nchunks = r.nchunks;
     a.l2_window = r.l2_window;
     a.b_bytes = sizeof(float) * (size_t)nc * nv;
-    a.list_mode = 2;  // the plan's fixed list of chunks with an empty row
+    carve_balanced(r, ws, ws_bytes, &a);
+    // the plan's chunk groups per call are those of its aligned operands
+    if (!win_aligned<float>(a, r.W == 32 ? 4 : 8)) return false;
+    const int nw = r.W == 128 ? 2 : 4;  // workers per warp
+    const unsigned long long ngroups = ((unsigned long long)r.nchunks + nw - 1) / nw;
     a.head_base = (unsigned int)(call * ngroups);  // claims of the calls before, mod 2^32
-    carve_balanced(r, ws, &a);
+    if (nempty > 0) {
+        const unsigned g = (unsigned)std::min<long long>(((long long)nempty + 7) / 8,
+                                                         (long long)device_sms() * 8);
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(g);
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_rows_beta, empty, nempty, C, nv, 0.0f);
+        count_launches(1);
+    }
     timer_before(st);
-    bool ok = false;
-    if (r.W == 128 && (ok = launch_grp<128, float, float>(r, a, st)))
-        launch_walk_list<128, float, float>(r, a, st);
-    else if (r.W == 64 && (ok = launch_grp<64, float, float>(r, a, st)))
-        launch_walk_list<64, float, float>(r, a, st);
+    launch_tma(r, a, st);
     timer_after(st);
-    if (ok) count_launches(1);
-    return ok;
+    count_launches(1);
+    return true;
 }
 
-void workspace_tables(const Resolved &r, void *ws, const int2 **meta, int **list)
+void carve_and_partition(const Resolved &r, int nr, int nnz, int nv, const int *rowPtr, void *ws,
+                         size_t ws_bytes, cudaStream_t st)
 {
     KArgs a{};
-    carve_balanced(r, ws, &a);
-    *meta = a.meta;
-    *list = a.list;
+    a.nv = nv;
+    carve_balanced(r, ws, ws_bytes, &a);
+    launch_partition(r, nr, nnz, rowPtr, a, false, st);
 }
 
-void carve_and_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, void *ws,
-                         cudaStream_t st)
-{
-    KArgs a{};
-    carve_balanced(r, ws, &a);
-    launch_partition(r, nr, nnz, rowPtr, a, st);
-}
-
-void carve_balanced(const Resolved &r, void *ws, KArgs *a)
+void carve_balanced(const Resolved &r, void *ws, size_t ws_bytes, KArgs *a)
 {
     char *p = (char *)ws;
     a->meta = (const int2 *)p;
@@ -514,13 +582,13 @@ void carve_balanced(const Resolved &r, void *ws, KArgs *a)
     p += align256(sizeof(int) * (size_t)r.nchunks * r.tiles);
     a->head = (unsigned int *)p;
     p += align256(sizeof(unsigned int) * (size_t)r.tiles);
-    a->list = (int *)p;
-    p += align256(sizeof(int) * ((size_t)r.nchunks + 1));
     a->slots = (float *)p;
+    const size_t least = workspace_least(r, a->nv), map = emap_bytes(r);
+    if (map && ws_bytes >= least + map) a->emap = (unsigned int *)((char *)ws + least);
 }
 
 void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, const KArgs &a,
-                      cudaStream_t st)
+                      bool rows_beta, cudaStream_t st)
 {
     // one thread per row (a grid-stride form over 2 or 4 CTAs per SM measured
     // equal or slower)
@@ -539,7 +607,7 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_partition, nr, nnz, rowPtr, (int)r.chunk, (int)r.snap,
                        (int)r.nchunks, const_cast<int2 *>(a.meta), a.cnt, (int)r.tiles, a.head,
-                       a.list);
+                       a.emap, rows_beta ? a.C : (float *)nullptr, a.nv, a.beta);
     count_launches(1);
 }
 
@@ -697,7 +765,7 @@ daspmm_status daspmm_partition(int nr, int nnz, const int *rowPtr, int chunk, in
     const unsigned pg = (unsigned)std::max(1, (nr + 255) / 256);
     k_partition<<<pg, 256, 0, (cudaStream_t)stream>>>(nr, nnz, rowPtr, chunk, std::min(snap, chunk),
                                                       nch, (int2 *)meta, nullptr, 1, nullptr,
-                                                      nullptr);
+                                                      nullptr, nullptr, 0, 0.0f);
     count_launches(1);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);

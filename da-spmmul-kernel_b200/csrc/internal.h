@@ -21,7 +21,8 @@ struct Resolved {
     int block, tiles;
     int pipe;  // balanced CSR: 1 register gather, 2 TMA ring, 3 cp.async ring, 4 lean
                // gather, 5 column-major through a row-major product (transposes)
-    int W;     // TMA ring: tile width in floats (32, 64, 128)
+    int W;     // pipes 2..4 and `general`: tile width in floats
+    int general;  // pipe 1, row-major: the masked window kernel's vector width (0: k_bal)
     int inner_chunk;  // pipe 5: the caller's chunk for the row-major product
     int l2_window;    // thousandths of B's lines marked L2-persisting (0 = off)
 };
@@ -52,7 +53,9 @@ daspmm_status cuda_fail(cudaError_t e);
 
 daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int nnz, int nv,
                       const void *B, const void *C, Resolved *out);
+// What a product asks for, and the least that it can do with.
 size_t workspace_bytes(const Resolved &r, int nv);
+size_t workspace_least(const Resolved &r, int nv);
 daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nnz, int nv,
                            const int *rowPtr, const int *rowIdx, const int *colIdx,
                            const float *values, const float *B, float *C, float beta,
@@ -60,27 +63,27 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
 // Balanced CSR: the workspace's boundary table, split-row counters, chunk
 // queue heads and carry slots, and the partition launch that fills them.
 struct KArgs;
-void carve_balanced(const Resolved &r, void *ws, KArgs *a);
+void carve_balanced(const Resolved &r, void *ws, size_t ws_bytes, KArgs *a);  // a->nv is set
+// `rows_beta`: the rows without nonzeros are finished by the partition (the
+// window kernel does not visit them).
 void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, const KArgs &a,
-                      cudaStream_t st);
+                      bool rows_beta, cudaStream_t st);
 // carve_balanced + launch_partition on a workspace (the boundaries and the
 // zeroed queue state of the balanced split).
-void carve_and_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, void *ws,
-                         cudaStream_t st);
+void carve_and_partition(const Resolved &r, int nr, int nnz, int nv, const int *rowPtr, void *ws,
+                         size_t ws_bytes, cudaStream_t st);
 daspmm_status cached_workspace(size_t need, cudaStream_t st, void **out);
-// A planned FP32 row-major balanced-CSR product (plan.cu): the worker-group
+// A planned FP32 row-major balanced-CSR product (plan.cu), beta == 0: the
 // window kernel alone, over a workspace whose chunk boundaries k_partition
-// wrote once (the kernel leaves its queue heads and split-row counters at
-// zero).  Returns false, launching nothing, when that kernel does not take
-// the call (beta != 0, alignment, tile width).
+// wrote once (the kernel leaves its split-row counters at zero), and the
+// `nempty` rows without nonzeros (device list `empty`).  False, launching
+// nothing, when the window kernel does not take the plan's configuration.
 // `call` counts the planned products since the boundaries were computed: a
 // call's window kernel makes exactly one queue claim per chunk group, so
 // each call counts its claims on from call x groups (no reset between calls).
 bool run_planned(const Resolved &r, int nr, int nc, int nnz, int nv, const int *rowPtr,
                  const int *colIdx, const float *values, const float *B, float *C, void *ws,
-                 unsigned long long call, cudaStream_t st);
-// The boundary table and the walk list inside a balanced-CSR workspace.
-void workspace_tables(const Resolved &r, void *ws, const int2 **meta, int **list);
+                 size_t ws_bytes, const int *empty, int nempty, unsigned long long call, cudaStream_t st);
 daspmm_status cached_host_staging(size_t need, cudaStream_t st, void **out);
 
 // Launch accounting and the optional event hook around main kernels.

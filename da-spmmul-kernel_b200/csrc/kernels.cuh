@@ -54,9 +54,7 @@ struct KArgs {
     int *cnt;           // pieces arrived per split row and column tile, at the
                         // row's first chunk: [nchunks][tiles]
     unsigned int *head; // chunks handed out per column tile [tiles]
-    int *list;          // chunks the fast kernel left to the walk: [0] count, then ids
-    int list_mode;      // walk kernel: 0 every chunk (queue), 1 the listed ones, 2 a
-                        // planned product's fixed list (window kernel: don't list)
+    unsigned int *emap;  // bit r: row r has no nonzeros (k_partition; null: not kept)
     unsigned int head_base;  // window kernel: queue claims counted from here
     const float *bscale;  // FP8 B: per-column scales
     int kahan_min;        // rows at least this long use compensated sums
@@ -552,25 +550,38 @@ __global__ void __launch_bounds__(256) k_fix_coo(const KArgs a)
 // in lanes; k_fix_bal adds the carries of rows longer than the snap
 // threshold that straddle chunk boundaries.
 // ======================================================================
+// The window kernel leaves rows without nonzeros to this pass: with C they are
+// finished here (C = beta*C, nv columns, the warp together), with emap their
+// bitmap is kept.
 static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowPtr,
                             int chunk, int snap, int nchunks, int2 *meta, int *cnt, int tiles,
-                            unsigned int *head, int *list)
+                            unsigned int *head, unsigned int *emap, float *C, int nv, float beta)
 {
     asm volatile("griddepcontrol.launch_dependents;");  // the gather may be scheduled now
     // launched as a programmatic dependent of the stream's previous kernel (the
-    // last SpMM's walk, say): nothing is read or written before it completes
+    // last SpMM's gather, say): nothing is read or written before it completes
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long r0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31;
     if (r0 == 0) {
         meta[0] = make_int2(0, 0);
         meta[nchunks] = make_int2(nnz, nr);
         if (head)
             for (int t = 0; t < tiles; ++t) head[t] = 0;
-        if (list) list[0] = 0;
     }
     const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long r = r0; r < nr; r += stride) {
-        const int rs = __ldg(rowPtr + r), re = __ldg(rowPtr + r + 1);
+    for (long long r = r0; r - lane < nr; r += stride) {
+        const int rs = r < nr ? __ldg(rowPtr + r) : 0, re = r < nr ? __ldg(rowPtr + r + 1) : 0;
+        unsigned none = __ballot_sync(kFull, r < nr && rs == re);
+        if (emap && lane == 0) emap[r >> 5] = none;
+        if (C) {
+            while (none) {
+                float *dst = C + (size_t)(r - lane + __ffs(none) - 1) * nv;
+                none &= none - 1;
+                for (int k = lane; k < nv; k += 32)
+                    dst[k] = beta == 0.0f ? 0.0f : fmaf(beta, dst[k], 0.0f);
+            }
+        }
         if (rs == re) continue;
         long long c = ((long long)rs + chunk - 1) / chunk;
         if (c < 1) c = 1;
@@ -585,6 +596,22 @@ static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowP
         // tile) live at its first chunk
         if (split && cnt)
             for (int t = 0; t < tiles; ++t) cnt[(size_t)(rs / chunk) * tiles + t] = 0;
+    }
+}
+
+// C = beta*C for `n` listed rows of nv columns, a warp per row: a planned
+// product's rows without nonzeros.
+static __global__ void __launch_bounds__(256)
+    k_rows_beta(const int *__restrict__ rows, int n, float *C, int nv, float beta)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int lane = threadIdx.x & 31;
+    for (long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < n;
+         i += ((long long)gridDim.x * blockDim.x) >> 5) {
+        float *dst = C + (size_t)__ldg(rows + i) * nv;
+        for (int k = lane; k < nv; k += 32)
+            dst[k] = beta == 0.0f ? 0.0f : fmaf(beta, dst[k], 0.0f);
     }
 }
 
@@ -638,26 +665,6 @@ __device__ __forceinline__ void piece_arrive(const KArgs &a, int row, int col, i
         for (int e = 0; e < VL; ++e) tot[e] = fmaf(a.beta, old[e], tot[e]);
     }
     st_v<VL>(dst, tot);
-}
-
-// piece_arrive out of line, for kernels whose main loop needs every register
-// (split rows are a small fraction of the rows).
-template <int VL>
-__device__ __noinline__ void piece_arrive_ool(const int *__restrict__ rowPtr, int *cnt,
-                                              const float *slots, float *C, int ldc, int nv,
-                                              int chunk, float beta, int row, int col,
-                                              int tiles, int tile)
-{
-    KArgs a{};
-    a.rowPtr = rowPtr;
-    a.cnt = cnt;
-    a.slots = const_cast<float *>(slots);
-    a.C = C;
-    a.ldc = ldc;
-    a.nv = nv;
-    a.chunk = chunk;
-    a.beta = beta;
-    piece_arrive<VL>(a, row, col, tiles, tile);
 }
 
 template <bool CM, int V, int CF, bool RECORD>

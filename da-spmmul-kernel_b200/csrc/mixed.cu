@@ -2,7 +2,7 @@
 // per-column scales, FP32 accumulation, optional Kahan rows) and the device
 // quantizers that produce its inputs.  No counterpart in the reference, whose
 // kernels are FP32 only (spmm.h:17-18); this extends that value/B type.
-#include "gather_lean.cuh"
+#include "gather_win.cuh"
 #include "internal.h"
 #include "kernels.cuh"
 
@@ -109,7 +109,7 @@ static __global__ void __launch_bounds__(256)
         if (t >= active) return;
         const int c = (int)(t % cvec) * 8;
 #pragma unroll
-        for (int e = 0; e < 8; ++e) sc[e] = __ldg(scale + c + e);
+        for (int e = 0; e < 8; ++e) sc[e] = __ldcg(scale + c + e);
     }
     auto one = [&](long long v, const float4 &a, const float4 &b) {
         float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -302,13 +302,13 @@ daspmm_status daspmm_spmm_mixed(const daspmm_config *cfg_in, int layout, int nr,
     if (nr == 0) return DASPMM_OK;
     if (!B || !C || !rowPtr || (nnz > 0 && (!colIdx || !values))) return DASPMM_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
-    const size_t need = workspace_bytes(r, nv);
     if (!workspace) {
+        const size_t need = workspace_bytes(r, nv);
         s = cached_workspace(need, st, &workspace);
         if (s != DASPMM_OK) return s;
         ws_bytes = need;
     }
-    if (need > ws_bytes) return DASPMM_ERR_WORKSPACE;
+    if (workspace_least(r, nv) > ws_bytes) return DASPMM_ERR_WORKSPACE;
 
     KArgs a{};
     a.nr = nr; a.nc = nc; a.nnz = nnz; a.nv = nv;
@@ -322,10 +322,10 @@ daspmm_status daspmm_spmm_mixed(const daspmm_config *cfg_in, int layout, int nr,
     a.kahan_min = kahan_min > 0 ? kahan_min : 0x7fffffff;
     a.l2_window = r.l2_window;
     a.b_bytes = (size_t)fmt_bytes(b_fmt) * nc * nv;
-    carve_balanced(r, workspace, &a);
-    launch_partition(r, nr, nnz, rowPtr, a, st);
-    timer_before(st);  // the optional timer brackets the main kernel
+    carve_balanced(r, workspace, ws_bytes, &a);
     const bool kahan = kahan_min > 0;
+    launch_partition(r, nr, nnz, rowPtr, a, !kahan, st);
+    timer_before(st);  // the optional timer brackets the main kernel
     if (val_fmt == DASPMM_F32 && b_fmt == DASPMM_F32) launch_mixed<float, float>(r, a, kahan, st);
     else if (val_fmt == DASPMM_BF16 && b_fmt == DASPMM_BF16) launch_mixed<bf16, bf16>(r, a, kahan, st);
     else if (val_fmt == DASPMM_F16) launch_mixed<fp16, fp16>(r, a, kahan, st);

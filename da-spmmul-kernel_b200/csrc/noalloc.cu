@@ -102,7 +102,7 @@ extern "C" daspmm_status daspmm_spmm_noalloc(int layout, int nr, int nc, int nnz
     daspmm_status s = daspmm::resolve(&cfg, layout, nr, nc, nnz, nv, B, C, &r);
     if (s != DASPMM_OK) return s;
     // Too large for the fixed scratch: refuse before touching the device.
-    if (daspmm::workspace_bytes(r, nv) > (size_t)DASPMM_NOALLOC_MAX_BYTES)
+    if (daspmm::workspace_least(r, nv) > (size_t)DASPMM_NOALLOC_MAX_BYTES)
         return DASPMM_ERR_WORKSPACE;
     void *scratch = nullptr;
     s = scratch_address(&scratch);

@@ -5,18 +5,18 @@
 // change the matrix between calls.  A caller that multiplies the same matrix
 // by many dense operands (an iterative solver, a GNN layer over one graph, a
 // serving loop over a resident matrix) can instead create a plan: the
-// boundaries, and the list of chunks with an empty row (which the walk kernel
-// sums), are computed once into a workspace the plan owns, and each product is
-// the worker-group window kernel plus the walk over that fixed list -- no
-// partition pass.  Between products nothing is reset: the split-row counters
-// return to zero by themselves (the last piece of a row clears its counter),
-// and each call counts its queue claims on from where the previous call's
-// ended (a call makes exactly one claim per chunk group).  Results are
-// bit-identical to daspmm_spmm with the same configuration (same chunks, same
-// order of summation).  Calls the window kernel does not take (beta != 0, B
-// or C not 32-byte aligned, tiles other than 128 or 64 columns) run the
-// stateless path on the plan's workspace, and the next planned call first
-// writes the boundaries and the list again.
+// boundaries, and the list of rows without nonzeros, are computed once into
+// memory the plan owns, and each product is the worker-group window kernel,
+// with no partition pass (and, where the matrix has rows without nonzeros, one
+// small launch that clears them).  Between products nothing is reset: the
+// split-row counters return to zero by themselves (the last piece of a row
+// clears its counter), and each call counts its queue claims on from where the
+// previous call's ended (a call makes exactly one claim per chunk group).
+// Results are bit-identical to daspmm_spmm with the same configuration (same
+// chunks, same order of summation).  Calls the planned form does not take
+// (beta != 0, B or C off the window kernel's alignment, widths that are no
+// multiple of 32) run the stateless path on the plan's workspace, and the next
+// planned call first writes the boundaries again.
 #include "internal.h"
 
 #include <cuda_runtime.h>
@@ -31,8 +31,9 @@ struct daspmm_plan_s {
     const float *values;
     void *ws = nullptr;
     size_t ws_bytes = 0;
-    std::vector<int> list;   // [count, chunk ids...]: chunks with an empty row
-    bool fresh = false;      // boundaries and list in the workspace are the plan's
+    int *empty = nullptr;    // device: the rows without nonzeros
+    int nempty = 0;
+    bool fresh = false;      // the boundaries in the workspace are the plan's
     unsigned long long calls = 0;  // planned products since they were written
     int dev = 0;
 };
@@ -40,50 +41,33 @@ struct daspmm_plan_s {
 namespace {
 
 // Boundaries (k_partition, which also zeroes the queue heads and split-row
-// counters) and the fixed walk list into the plan's workspace.
-daspmm_status refresh(daspmm_plan p, cudaStream_t st)
+// counters) into the plan's workspace.
+void refresh(daspmm_plan p, cudaStream_t st)
 {
-    daspmm::carve_and_partition(p->r, p->nr, p->nnz, p->rowPtr, p->ws, st);
-    const int2 *meta = nullptr;
-    int *list = nullptr;
-    daspmm::workspace_tables(p->r, p->ws, &meta, &list);
-    cudaError_t e = cudaMemcpyAsync(list, p->list.data(), sizeof(int) * p->list.size(),
-                                    cudaMemcpyHostToDevice, st);
-    if (e != cudaSuccess) return daspmm::cuda_fail(e);
+    daspmm::carve_and_partition(p->r, p->nr, p->nnz, p->nv, p->rowPtr, p->ws, p->ws_bytes, st);
     p->fresh = true;
     p->calls = 0;
-    return DASPMM_OK;
 }
 
-// The chunks whose rows [s_c, s_{c+1}) hold an empty row: the window kernel
-// cannot sum them (a bitmask of row ends cannot express two rows ending at
-// one position), the walk kernel does.  Same rule as the window kernel's.
-daspmm_status build_list(daspmm_plan p, cudaStream_t st)
+// The rows without nonzeros, which the window kernel does not visit, from the
+// row pointer (read once on the host).
+daspmm_status list_empty_rows(daspmm_plan p, cudaStream_t st)
 {
-    const int nch = p->r.nchunks;
-    std::vector<int2> meta((size_t)nch + 1);
-    std::vector<int> rp((size_t)p->nr + 1);
-    const int2 *d_meta = nullptr;
-    int *d_list = nullptr;
-    daspmm::workspace_tables(p->r, p->ws, &d_meta, &d_list);
-    daspmm::carve_and_partition(p->r, p->nr, p->nnz, p->rowPtr, p->ws, st);
-    cudaError_t e = cudaMemcpyAsync(meta.data(), d_meta, sizeof(int2) * meta.size(),
+    std::vector<int> rp((size_t)p->nr + 1), list;
+    cudaError_t e = cudaMemcpyAsync(rp.data(), p->rowPtr, sizeof(int) * rp.size(),
                                     cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(rp.data(), p->rowPtr, sizeof(int) * rp.size(),
-                            cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return daspmm::cuda_fail(e);
-    p->list.assign(1, 0);
-    for (int c = 0; c < nch; ++c) {
-        for (int r = meta[c].y; r < meta[c + 1].y; ++r) {
-            if (rp[r] == rp[r + 1]) {
-                p->list.push_back(c);
-                break;
-            }
-        }
-    }
-    p->list[0] = (int)p->list.size() - 1;
+    for (int r = 0; r < p->nr; ++r)
+        if (rp[r] == rp[r + 1]) list.push_back(r);
+    if (list.empty()) return DASPMM_OK;
+    e = cudaMalloc(&p->empty, sizeof(int) * list.size());
+    if (e == cudaSuccess)
+        e = cudaMemcpyAsync(p->empty, list.data(), sizeof(int) * list.size(),
+                            cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) return daspmm::cuda_fail(e);
+    p->nempty = (int)list.size();
     return DASPMM_OK;
 }
 
@@ -121,14 +105,15 @@ daspmm_status daspmm_plan_create(const daspmm_config *cfg, int nr, int nc, int n
         }
     }
     if (r.pipe == 4 && nr > 0) {
-        s = build_list(p, st);
-        if (s == DASPMM_OK) s = refresh(p, st);
+        s = list_empty_rows(p, st);
         if (s == DASPMM_OK) {
+            refresh(p, st);
             cudaError_t e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) s = daspmm::cuda_fail(e);
         }
         if (s != DASPMM_OK) {
             cudaFree(p->ws);
+            cudaFree(p->empty);
             delete p;
             return s;
         }
@@ -144,19 +129,16 @@ daspmm_status daspmm_plan_spmm(daspmm_plan p, const float *B, float *C, float be
     if (!B || !C) return DASPMM_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
     if (beta == 0.0f && p->r.pipe == 4) {
-        if (!p->fresh) {
-            daspmm_status s = refresh(p, st);
-            if (s != DASPMM_OK) return s;
-        }
+        if (!p->fresh) refresh(p, st);
         if (daspmm::run_planned(p->r, p->nr, p->nc, p->nnz, p->nv, p->rowPtr, p->colIdx,
-                                p->values, B, C, p->ws, p->calls, st)) {
+                                p->values, B, C, p->ws, p->ws_bytes, p->empty, p->nempty, p->calls, st)) {
             ++p->calls;
             cudaError_t e = cudaGetLastError();
             return e == cudaSuccess ? DASPMM_OK : daspmm::cuda_fail(e);
         }
     }
-    // the stateless path on the plan's workspace: it rewrites the boundaries,
-    // the queue heads and the list, so the next planned call refreshes them
+    // the stateless path on the plan's workspace: it rewrites the boundaries
+    // and the queue heads, so the next planned call refreshes them
     p->fresh = false;
     return daspmm::run_resolved(p->r, DASPMM_ROW_MAJOR, p->nr, p->nc, p->nnz, p->nv, p->rowPtr,
                                 nullptr, p->colIdx, p->values, B, C, beta, p->ws, p->ws_bytes,
@@ -177,6 +159,8 @@ daspmm_status daspmm_plan_destroy(daspmm_plan p)
     cudaGetDevice(&cur);
     if (cur != p->dev) cudaSetDevice(p->dev);
     cudaError_t e = p->ws ? cudaFree(p->ws) : cudaSuccess;
+    const cudaError_t e2 = p->empty ? cudaFree(p->empty) : cudaSuccess;
+    if (e == cudaSuccess) e = e2;
     if (cur != p->dev) cudaSetDevice(cur);
     delete p;
     return e == cudaSuccess ? DASPMM_OK : daspmm::cuda_fail(e);

@@ -430,9 +430,11 @@ daspmm_status daspmm_spmm_host_async(const daspmm_config *cfg, int layout, int n
  * rowPtr / colIdx / values, which must stay unchanged and alive until
  * daspmm_plan_destroy), row-major layout and nv: the boundaries are computed
  * once, into a workspace the plan owns, and each daspmm_plan_spmm with beta
- * == 0 and B / C 32-byte aligned is one launch of the window kernel.  Results
+ * == 0, nv a multiple of 32 and B / C 32-byte aligned is one launch of the
+ * window kernel (and one of a kernel that clears them, where the matrix has
+ * rows without nonzeros).  Results
  * are bit-identical to daspmm_spmm with the plan's configuration.  Other calls
- * (beta != 0, other alignment) take the stateless path on the plan's
+ * (beta != 0, other widths or alignment) take the stateless path on the plan's
  * workspace.  cfg: NULL or {.alg = DASPMM_ALG_CSR_BALANCED, ...}.
  * daspmm_plan_create allocates (cudaMalloc) and synchronises `stream`.
  * Calls on one plan share its workspace: order them (one stream); calls that
