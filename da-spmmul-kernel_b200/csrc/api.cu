@@ -11,6 +11,7 @@
 #include "kernels.cuh"
 #include "gather_tma.cuh"
 #include "gather_win.cuh"
+#include "gather_stream.cuh"
 #include "internal.h"
 
 #include <cuda_runtime.h>
@@ -192,15 +193,17 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
     const int G = r.L * r.S;
     // every field of the shape is zero or what zero would give
     daspmm_config d = *cfg;
-    const bool plain_shape = (!d.vec || d.vec == default_vec(nv, B, C)) &&
-                             (!d.cf || d.cf == (vecs > 32 ? 2 : 1)) &&
-                             (!d.lanes_col || d.lanes_col == std::min(32, pow2ceil((vecs + r.CF - 1) / r.CF)));
+    const bool plain_shape =
+        (!d.vec || d.vec == (r.cm ? 1 : default_vec(nv, B, C))) &&
+        (!d.cf || d.cf == (r.cm ? std::min(8, pow2ceil(nv)) : vecs > 32 ? 2 : 1)) &&
+        (!d.lanes_col ||
+         d.lanes_col == (r.cm ? 1 : std::min(32, pow2ceil((vecs + r.CF - 1) / r.CF))));
     // chunks
     if (cfg->alg >= DASPMM_ALG_COO_SCALAR) {
         if (cfg->chunk) r.chunk = cfg->chunk;
         else if (cfg->alg == DASPMM_ALG_COO_VECTOR) r.chunk = std::max(64, 8 * r.S);
         else if (r.cm) r.chunk = 32;
-        else r.chunk = G >= 32 ? 128 : (G >= 16 || (!r.cm && nv > 16) ? 64 : 32);
+        else r.chunk = G >= 32 ? 128 : (G >= 16 || (!r.cm && nv > kStreamMaxNv) ? 64 : 32);
         if (r.chunk < 1) return DASPMM_ERR_INVALID;
         if (cfg->alg == DASPMM_ALG_COO_VECTOR && r.chunk % r.S) return DASPMM_ERR_INVALID;
         r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
@@ -247,7 +250,17 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
             }
         }
     }
-    if (r.pipe == 1 && cfg->alg == DASPMM_ALG_CSR_BALANCED && !r.cm && nv > 16 && plain_shape) {
+    if (r.pipe == 1 && cfg->alg == DASPMM_ALG_CSR_BALANCED && nv <= kStreamMaxNv && plain_shape &&
+        !(r.cm && cfg->pipe == 1 && !cfg->chunk) &&
+        (!cfg->chunk || (cfg->chunk % 128 == 0 && cfg->chunk <= stream_chunk_most(nv))) &&
+        (!cfg->snap || cfg->snap == kStreamSnap)) {
+        r.stream = r.V;
+        r.chunk = cfg->chunk ? cfg->chunk : stream_chunk(nnz, nv);
+        r.snap = kStreamSnap;
+        r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
+        r.block = 256;
+    } else if (r.pipe == 1 && cfg->alg == DASPMM_ALG_CSR_BALANCED && !r.cm && nv > kStreamMaxNv &&
+               plain_shape) {
         // the shape is the library's: the window kernel with masked columns
         r.general = r.V;
         r.W = general_width(r.V, nv);
@@ -290,10 +303,15 @@ size_t workspace_least(const Resolved &r, int nv)
     if (r.pipe == 5) {  // [B row-major | C row-major | the row-major product's own]
         Resolved in;
         if (resolve_inner(r, nv, nullptr, nullptr, &in) != DASPMM_OK) return 0;
+        // (k_stream stores C column-major itself)
         return align256(sizeof(float) * (size_t)r.nc * nv) +
-               align256(sizeof(float) * (size_t)r.nr * nv) + workspace_bytes(in, nv);
+               (in.stream ? 0 : align256(sizeof(float) * (size_t)r.nr * nv)) +
+               workspace_bytes(in, nv);
     }
     size_t b = 0;
+    if (r.stream)  // boundaries, slots of cut rows
+        return align256(sizeof(int2) * ((size_t)r.nchunks + 1)) +
+               align256(sizeof(float) * 2 * (size_t)r.nchunks * nv);
     if (r.alg == DASPMM_ALG_CSR_BALANCED) {
         b += align256(sizeof(int2) * ((size_t)r.nchunks + 1));
         b += align256(sizeof(int) * (size_t)r.nchunks * r.tiles);  // split-row arrival counters
@@ -454,6 +472,31 @@ static unsigned grid_x(long long units, int G, int block)
     return (unsigned)g;
 }
 
+// k_stream on a workspace of workspace_least bytes; cmb / cmc: B / C column-major.
+static void run_stream(const Resolved &r, bool cmb, bool cmc, int nr, int nc, int nnz, int nv,
+                       const int *rowPtr, const int *colIdx, const float *values, const float *B,
+                       float *C, float beta, void *ws, cudaStream_t st)
+{
+    KArgs a{};
+    a.nr = nr; a.nc = nc; a.nnz = nnz; a.nv = nv;
+    a.ldb = cmb ? nc : nv;
+    a.ldc = cmc ? nr : nv;
+    a.rowPtr = rowPtr; a.colIdx = colIdx; a.vals = values;
+    a.B = B; a.C = C; a.beta = beta;
+    a.chunk = r.chunk; a.nchunks = r.nchunks;
+    a.meta = (const int2 *)ws;
+    a.slots = (float *)((char *)ws + align256(sizeof(int2) * ((size_t)r.nchunks + 1)));
+    if (nv == 1) {  // one column has no layout
+        cmb = cmc = false;
+        a.ldb = a.ldc = 1;
+    }
+    timer_before(st);
+    if (cmc) launch_stream<true>(r.stream, cmb, a, st);
+    else launch_stream<false>(r.stream, cmb, a, st);
+    timer_after(st);
+    count_launches(r.nchunks > 1 ? 2 : 1);
+}
+
 daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nnz, int nv,
                            const int *rowPtr, const int *rowIdx, const int *colIdx,
                            const float *values, const float *B, float *C, float beta,
@@ -477,10 +520,23 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
         if (s != DASPMM_OK) return s;
         // B column-major = an nv x nc row-major array; its transpose is row-major B
         launch_transpose(B, nv, nc, Brm, 0.0f, st);
+        if (in.stream) {
+            run_stream(in, false, true, nr, nc, nnz, nv, rowPtr, colIdx, values, Brm, C, beta, Crm,
+                       st);
+            const cudaError_t e = cudaGetLastError();
+            return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
+        }
         s = run_resolved(in, DASPMM_ROW_MAJOR, nr, nc, nnz, nv, rowPtr, rowIdx, colIdx, values,
                          Brm, Crm, 0.0f, iws, workspace_bytes(in, nv), st);
         if (s != DASPMM_OK) return s;
         launch_transpose(Crm, nr, nv, C, beta, st);  // C = transpose + beta * C
+        const cudaError_t e = cudaGetLastError();
+        return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
+    }
+
+    if (r.stream) {
+        const bool cm = layout == DASPMM_COL_MAJOR;
+        run_stream(r, cm, cm, nr, nc, nnz, nv, rowPtr, colIdx, values, B, C, beta, ws, st);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
     }
@@ -623,7 +679,8 @@ struct WsKey {
         return tag < o.tag;
     }
 };
-static std::mutex g_ws_mu;
+static std::recursive_mutex g_ws_mu;
+std::recursive_mutex &workspace_mutex() { return g_ws_mu; }
 static std::map<WsKey, std::pair<void *, size_t>> g_ws;
 
 static daspmm_status cached_block(size_t need, cudaStream_t st, int tag, void **out)
@@ -633,7 +690,7 @@ static daspmm_status cached_block(size_t need, cudaStream_t st, int tag, void **
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e);
-    std::lock_guard<std::mutex> lk(g_ws_mu);
+    std::lock_guard<std::recursive_mutex> lk(g_ws_mu);
     auto &slot = g_ws[WsKey{dev, (void *)st, tag}];
     if (slot.second < need) {
         if (slot.first) {
@@ -708,7 +765,9 @@ daspmm_status daspmm_spmm_ex(const daspmm_config *cfg, int layout, int nr, int n
     daspmm_status s = resolve(cfg, layout, nr, nc, nnz, nv, B, C, &r);
     if (s != DASPMM_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
+    std::unique_lock<std::recursive_mutex> hold(workspace_mutex(), std::defer_lock);
     if (!workspace) {
+        hold.lock();
         const size_t need = workspace_bytes(r, nv);
         s = cached_workspace(need, st, &workspace);
         if (s != DASPMM_OK) return s;

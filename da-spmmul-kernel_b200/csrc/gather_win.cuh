@@ -262,6 +262,7 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
             clear();
             cont = false;
         };
+        bool sought = false;
         for (; nwin > 0; --nwin) {
             const int left = ke - wb;  // <= 0: this worker is done
             int wlen = G;              // (without gaps; a worker's last window may hold fewer)
@@ -275,11 +276,14 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
                 const int f = __ffs(~live | (1u << (G - 1) << 1)) - 1;  // rows r .. r + f - 1
                 const int Ef = __shfl_sync(kFull, E, max(0, f - 1), G);
                 wlen = f > 0 ? max(0, min(min(G, left), Ef - wb)) : 0;
+                // (a row pointer that does not ascend must not hold the loop up)
+                if (sought && wlen == 0) wlen = min(1, max(0, left));
                 if (gl >= wlen) {  // not this window's
                     ccur = 0;
                     vcur = 0.0f;
                 }
-                bool seek = left > 0 && f == 0;  // row r is empty: where is nonzero wb?
+                bool seek = wlen == 0 && left > 0;  // row r is empty: where is nonzero wb?
+                sought = seek;
                 if (__any_sync(kFull, seek)) {
                     const int near = __ffs(live) - 1;  // in sight
                     int lo = near >= 0 ? r + near : min(r + G, a.nr), hi = s1;
@@ -287,7 +291,7 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
                     while (__any_sync(kFull, far)) {
                         const int step = (hi - lo + G) / G, x = lo + gl * step;
                         const bool le = far && x <= hi && __ldg(a.rowPtr + x) <= wb;
-                        const int m = __popc(__ballot_sync(kFull, le) & gmask);
+                        const int m = max(1, __popc(__ballot_sync(kFull, le) & gmask));
                         if (far) {
                             lo += (m - 1) * step;
                             hi = min(hi, lo + step - 1);
@@ -296,7 +300,7 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
                     }
                     if (seek) r = lo;
                 }
-                if (f > 0 && wlen == Ef - wb) skip = max(0, __ffs(live >> f) - 1);
+                if (f > 0 && wlen > 0 && wlen == Ef - wb) skip = max(0, __ffs(live >> f) - 1);
                 nwin = 1 + (max(0, left - wlen) + G - 1) / G;
 #pragma unroll
                 for (int o = G; o < 32; o <<= 1)

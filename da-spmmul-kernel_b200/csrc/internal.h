@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 #include <stddef.h>
 
+#include <mutex>
 #include <vector>
 
 namespace daspmm {
@@ -22,6 +23,7 @@ struct Resolved {
     int pipe;  // balanced CSR: 1 register gather, 2 TMA ring, 3 cp.async ring, 4 lean
                // gather, 5 column-major through a row-major product (transposes)
     int W;     // pipes 2..4 and `general`: tile width in floats
+    int stream;   // few columns (k_stream): floats per access of B, 0: another kernel
     int general;  // pipe 1, row-major: the masked window kernel's vector width (0: k_bal)
     int inner_chunk;  // pipe 5: the caller's chunk for the row-major product
     int l2_window;    // thousandths of B's lines marked L2-persisting (0 = off)
@@ -72,6 +74,10 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
 // zeroed queue state of the balanced split).
 void carve_and_partition(const Resolved &r, int nr, int nnz, int nv, const int *rowPtr, void *ws,
                          size_t ws_bytes, cudaStream_t st);
+// The library's workspace of (device, stream).  A caller holds the lock from before
+// it asks until its kernels are queued: another thread's larger request waits for
+// the stream before it frees the block.
+std::recursive_mutex &workspace_mutex();
 daspmm_status cached_workspace(size_t need, cudaStream_t st, void **out);
 // A planned FP32 row-major balanced-CSR product (plan.cu), beta == 0: the
 // window kernel alone, over a workspace whose chunk boundaries k_partition

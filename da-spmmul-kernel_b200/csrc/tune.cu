@@ -132,6 +132,7 @@ std::vector<daspmm_config> candidates(int layout, int nv, bool have_coo)
         add(DASPMM_ALG_CSR_BALANCED, 2);
         add(DASPMM_ALG_CSR_BALANCED, 1);
     } else {
+        add(DASPMM_ALG_CSR_BALANCED);
         for (int ch : {32, 128}) add(DASPMM_ALG_CSR_BALANCED, 1, ch);
         if (layout == DASPMM_ROW_MAJOR && nv <= 8) {
             add(DASPMM_ALG_CSR_VECTOR, 0, 0, 4);
@@ -190,12 +191,11 @@ daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_c
             return DASPMM_OK;
         }
     }
-    // Rule of thumb for untuned shapes: the balanced split for wide dense
-    // operands (B rows of >= 128 bytes), the row-balanced scalar kernel
-    // otherwise.
+    // Untuned shapes: the balanced split, the fastest at every width and layout
+    // that was measured (k_stream up to 16 columns, the window kernel above,
+    // through transposes for column-major operands).
     daspmm_config c{};
-    c.alg = (layout == DASPMM_ROW_MAJOR && nv >= 32) ? DASPMM_ALG_CSR_BALANCED
-                                                      : DASPMM_ALG_CSR_SCALAR;
+    c.alg = DASPMM_ALG_CSR_BALANCED;
     Resolved r;
     daspmm_status s = resolve(&c, layout, nr, nc, nnz, nv, nullptr, nullptr, &r);
     if (s != DASPMM_OK) return s;

@@ -1,0 +1,80 @@
+"""Products of few columns (k_stream): chunk and row boundaries, rows cut once and
+many times, empty rows, both layouts, beta, addresses off the vectors, non-finite
+operands."""
+import numpy as np
+import pytest
+
+import daspmm as D
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _csr(lens, nc, seed):
+    rng = np.random.default_rng(seed)
+    rp = np.concatenate([[0], np.cumsum(lens)]).astype(np.int32)
+    ci = np.concatenate([np.sort(rng.choice(nc, int(k), replace=False)) for k in lens]
+                        + [np.zeros(0, int)]).astype(np.int32)
+    return D.Csr(len(lens), nc, rp, ci, rng.uniform(-1, 1, int(rp[-1])).astype(np.float32))
+
+
+@pytest.fixture(scope="module")
+def mats(cuda):
+    rng = np.random.default_rng(2)
+    short = rng.integers(0, 9, 3000)
+    cut = rng.integers(0, 4, 400)                 # rows around the lengths that are cut or
+    cut[::7] = rng.choice([62, 63, 64, 65, 95, 96, 97, 127, 128, 129, 200], cut[::7].size)
+    hub = rng.integers(0, 3, 300)
+    hub[[0, 150, 299]] = (5000, 1500, 700)        # over many chunks, first and last row too
+    empty = np.zeros(4000, int)
+    empty[[17, 2000, 3998]] = (1, 700, 3)
+    out = {"short": _csr(short, 900, 1), "cut": _csr(cut, 900, 2), "hub": _csr(hub, 6000, 3),
+           "empty": _csr(empty, 900, 4), "one": _csr([1], 1, 5)}
+    return {k: (A, D.DeviceCsr(A)) for k, A in out.items()}
+
+
+def _run(A, dA, alg, layout, nv, beta, off=0, cfg=None, bad=None):
+    import torch
+    rng = np.random.default_rng(nv)
+    B = rng.uniform(-1, 1, A.nc * nv).astype(np.float32)
+    if bad is not None:
+        B[:: 2 * nv + 1] = bad
+    C0 = rng.uniform(-1, 1, A.nr * nv).astype(np.float32)
+    Bt, Ct = (torch.zeros(x.size + 8, device="cuda")[off:off + x.size] for x in (B, C0))
+    Bt.copy_(torch.from_numpy(B))
+    Ct.copy_(torch.from_numpy(C0))
+    D.spmm(alg, layout, dA, Bt, Ct, beta=beta, nv=nv, cfg=cfg)
+    return B, C0, Ct.cpu().numpy()
+
+
+def _check(A, layout, nv, beta, B, C0, C):
+    c64, absc = O.spmm_f64(layout, A.nr, A.nc, A.rowPtr, A.colIdx, A.values, B, nv)
+    assert O.rel_err(C, c64 + beta * C0.astype(np.float64),
+                     absc + abs(beta) * np.abs(C0)) <= O.REL_TOL_F32
+
+
+@pytest.mark.parametrize("name", ["short", "cut", "hub", "empty", "one"])
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("nv", [1, 2, 3, 4, 5, 6, 7, 8, 9, 12, 16])
+def test_few_columns(mats, name, layout, nv):
+    A, dA = mats[name]
+    for beta in (0.0, 0.5):
+        for off in (0, 1, 2):
+            _check(A, layout, nv, beta, *_run(A, dA, 4, layout, nv, beta, off))
+    for chunk in (128, 256):   # an explicit chunk of the same kernel
+        _check(A, layout, nv, 0.0,
+               *_run(A, dA, 4, layout, nv, 0.0, cfg=D.Config(alg=4, chunk=chunk)))
+
+
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+def test_not_finite(mats, bad):
+    for name in ("short", "hub"):
+        A, dA = mats[name]
+        for layout in (0, 1):
+            for nv in (1, 3, 4, 8):
+                B, _, C = _run(A, dA, 4, layout, nv, 0.0, bad=bad)
+                want = O.spmm_f32(layout, A.nr, A.nc, A.rowPtr, A.colIdx, A.values, B, nv)
+                np.testing.assert_array_equal(np.isfinite(C), np.isfinite(want))
+                odd = ~np.isfinite(want)
+                np.testing.assert_array_equal(C[odd], want[odd])
+
