@@ -723,6 +723,87 @@ daspmm_status cached_host_staging(size_t need, cudaStream_t st, void **out)
     return cached_block(need, st, 1, out);
 }
 
+// A block of the cached workspace without an error where there is none: not when it
+// would have to grow beyond `most`, without memory, or inside a stream capture (a
+// graph would keep the address of a block that a later call may replace).
+static bool spare_workspace(size_t need, size_t most, cudaStream_t st, void **out)
+{
+    int dev = 0;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
+        cap != cudaStreamCaptureStatusNone) {
+        cudaGetLastError();
+        return false;
+    }
+    auto it = g_ws.find(WsKey{dev, (void *)st, 0});
+    if ((it == g_ws.end() || it->second.second < need) && need > most) return false;
+    return cached_workspace(need, st, out) == DASPMM_OK;
+}
+
+// A product asked for by one of the reference's four algorithms, none of whose
+// shape the caller chose, runs as the balanced one with the same meaning (sorted
+// rows; COO first makes its row pointer): it is the faster one at every width and
+// layout.  Measured (us, CSR scalar / CSR vector / COO scalar / COO vector -> balanced,
+// COO's conversion included, 262k power-law matrix): 
+//   row-major N = 1   322 / 56 / 79 / 27 -> 16 (COO 22)      4   308 / 88 / 86 / 33 -> 22 (30)
+//            32   359 / 166 / 168 / 135 -> 35 (68)       128  681 / 550 / 380 / 438 -> 83 (124)
+//   col-major  16   876 / 338 / 341 / 168 -> 55 (64)      128 2364 / 2618 / 1470 / 1125 -> 178 (218)
+// (uniform-random rows, row-major, N = 4 / 16 / 32: CSR scalar 18 / 31 / 66 -> 21 / 34 / 38.)
+// Not (done stays false) where it lacks workspace: column-major operands need copies
+// of B and C, and this library's own block is not grown past kSpareMost for them.
+constexpr size_t kSpareMost = (size_t)2 << 30;
+static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int nnz, int nv,
+                                      const int *rowPtr, const int *rowIdx, const int *colIdx,
+                                      const float *values, const float *B, float *C, float beta,
+                                      cudaStream_t st, bool *done)
+{
+    *done = false;
+    if (alg < DASPMM_ALG_CSR_SCALAR || alg > DASPMM_ALG_COO_VECTOR) return DASPMM_OK;
+    const bool coo = alg >= DASPMM_ALG_COO_SCALAR;
+    // what its own kernels refuse or answer without work stays with them
+    if (nr <= 0 || nnz <= 0 || nc <= 0 || !B || !C || !colIdx || !values ||
+        !(coo ? rowIdx : rowPtr))
+        return DASPMM_OK;
+    daspmm_config c{};
+    Resolved r;
+    c.alg = alg;
+    if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
+    c.alg = DASPMM_ALG_CSR_BALANCED;
+    if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
+    const size_t rows = coo ? align256(sizeof(int) * ((size_t)nr + 1)) : 0;
+    const size_t need = workspace_bytes(r, nv);
+    std::lock_guard<std::recursive_mutex> hold(g_ws_mu);
+    void *ws = nullptr;
+    if (!spare_workspace(rows + need, kSpareMost, st, &ws)) return DASPMM_OK;
+    char *own = (char *)ws + rows;
+    if (coo) {
+        // where the row-major product's boundaries will lie (k_stream keeps none)
+        Resolved in = r;
+        char *bounds = own;
+        if (r.pipe == 5) {
+            if (resolve_inner(r, nv, nullptr, nullptr, &in) != DASPMM_OK) return DASPMM_OK;
+            bounds += align256(sizeof(float) * (size_t)nc * nv) +
+                      align256(sizeof(float) * (size_t)nr * nv);
+        }
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(((long long)nnz + 1 + 255) / 256));
+        cfg.blockDim = dim3(256);
+        cfg.stream = st;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        cudaLaunchKernelEx(&cfg, k_coo_rows, nr, nnz, rowIdx, (int *)ws, (int)in.chunk,
+                           in.stream ? (int2 *)nullptr : (int2 *)bounds);
+        count_launches(1);
+        rowPtr = (const int *)ws;
+    }
+    *done = true;
+    return run_resolved(r, layout, nr, nc, nnz, nv, rowPtr, nullptr, colIdx, values, B, C, beta,
+                        own, need, st);
+}
+
 }  // namespace daspmm
 
 using namespace daspmm;
@@ -788,6 +869,11 @@ daspmm_status daspmm_spmm(int alg, int layout, int nr, int nc, int nnz, int nv,
         if (s != DASPMM_OK) return s;
     } else {
         c.alg = alg;
+        bool done = false;
+        const daspmm_status s = through_balanced(alg, layout, nr, nc, nnz, nv, rowPtr, rowIdx,
+                                                 colIdx, values, B, C, beta, (cudaStream_t)stream,
+                                                 &done);
+        if (done) return s;
     }
     return daspmm_spmm_ex(&c, layout, nr, nc, nnz, nv, rowPtr, rowIdx, colIdx, values, B, C,
                           beta, nullptr, 0, stream);

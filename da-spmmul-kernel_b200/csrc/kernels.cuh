@@ -903,6 +903,22 @@ static __global__ void k_coo_to_csr(int nr, int nnz, const int *__restrict__ row
     for (int r = prev + 1; r <= cur && r <= nr; ++r) rowPtr[r] = (int)p;
 }
 
+// The same, and boundaries that are in range whatever the rows are (k_partition
+// writes the balanced split's over them; of rows that do not ascend it would leave
+// some unwritten).  Launched as a dependent of the stream's previous kernel.
+static __global__ void k_coo_rows(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr,
+                                  int chunk, int2 *meta)
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (p > nnz) return;
+    const int prev = p == 0 ? -1 : __ldg(rowIdx + p - 1);
+    const int cur = p == nnz ? nr : __ldg(rowIdx + p);
+    for (int r = prev + 1; r <= cur && r <= nr; ++r) rowPtr[r] = (int)p;
+    if (meta && p < nnz && p % chunk == 0) meta[p / chunk] = make_int2((int)p, cur);
+}
+
 // Ownership recording buffers (tests): owner = INT_MAX / pieces = 0, then
 // unowned rows back to -1 after the walk.
 static __global__ void k_own_init(int *own, int nr)

@@ -1,6 +1,7 @@
-"""Products of few columns (k_stream): chunk and row boundaries, rows cut once and
-many times, empty rows, both layouts, beta, addresses off the vectors, non-finite
-operands."""
+"""Products of few columns (k_stream) and the reference's algorithms run as the
+balanced product: chunk and row boundaries, rows cut once and many times, empty
+rows, both layouts, beta, addresses off the vectors, non-finite operands, and the
+calls that keep their own kernels (stream capture, no room for the workspace)."""
 import numpy as np
 import pytest
 
@@ -78,3 +79,57 @@ def test_not_finite(mats, bad):
                 odd = ~np.isfinite(want)
                 np.testing.assert_array_equal(C[odd], want[odd])
 
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("nv", [1, 4, 16, 32, 41, 128])
+def test_reference_algorithms_are_the_balanced_product(mats, layout, nv):
+    for name in ("short", "hub", "empty"):
+        A, dA = mats[name]
+        for beta in (0.0, 1.0, 0.5):
+            want = _run(A, dA, 4, layout, nv, beta)[2]
+            for alg in range(4):
+                np.testing.assert_array_equal(_run(A, dA, alg, layout, nv, beta)[2], want)
+
+
+def test_inside_a_capture_they_keep_their_own_kernels(mats):
+    """A captured CSR call uses no workspace, so the graph stays good whatever later
+    calls do with the library's."""
+    import torch
+    A, dA = mats["short"]
+    st = torch.cuda.Stream()
+    for layout in (0, 1):
+        nv = 16
+        B = torch.rand(A.nc * nv, device="cuda")
+        C = torch.empty(A.nr * nv, device="cuda")
+        torch.cuda.synchronize()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            D.spmm(D.Alg.CSR_SCALAR, layout, dA, B, C, nv=nv, stream=st)
+        big = D.DeviceCsr(D.gen_uniform(20000, 20000, 8, seed=1))
+        Bb, Cb = (torch.zeros(20000 * 128, device="cuda") for _ in range(2))
+        D.spmm(D.Alg.CSR_BALANCED, layout, big, Bb, Cb, nv=128, stream=st)
+        C.fill_(float("nan"))
+        torch.cuda.synchronize()
+        g.replay()
+        torch.cuda.synchronize()
+        c64, absc = O.spmm_f64(layout, A.nr, A.nc, A.rowPtr, A.colIdx, A.values, B.cpu().numpy(), nv)
+        assert O.rel_err(C.cpu().numpy(), c64, absc) <= O.REL_TOL_F32
+
+
+def test_no_room_for_copies(cuda):
+    """Column-major operands whose copies would take more than the library keeps."""
+    import torch
+    n, nv = 3_000_000, 96
+    rows = np.arange(0, n, 3000)
+    lens = np.zeros(n, np.int64)
+    lens[rows] = 1
+    A = D.Csr(n, n, np.concatenate([[0], np.cumsum(lens)]).astype(np.int32),
+              rows.astype(np.int32), np.full(rows.size, 2.0, np.float32))
+    dA = D.DeviceCsr(A)
+    B = torch.rand(nv, n, device="cuda")
+    C = torch.full((nv, n), 3.0, device="cuda")
+    D.spmm(D.Alg.CSR_VECTOR, 1, dA, B, C, nv=nv)
+    want = torch.zeros(nv, n, device="cuda")
+    at = torch.from_numpy(rows).cuda()
+    want[:, at] = 2.0 * B[:, at]
+    assert torch.equal(C, want)
