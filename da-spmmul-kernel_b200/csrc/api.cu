@@ -114,6 +114,22 @@ static int general_width(int V, int nv)
     return per <= 96 ? 96 : 128;
 }
 
+// Nonzeros per chunk of the window kernel for a tile of W columns: `most`, or fewer
+// where that would leave resident workers without a chunk, but no fewer than 48
+// (shorter chunks cut more rows: power-law 30k rows, N = 128, 23.7 us at 48, 29.5 at 32).
+// Narrow tiles, whose workers run four to a warp, want a little over one chunk per
+// worker.  us at the chosen chunk against `most`: uniform 4k x 16, N = 32 / 128 / 512 8.6 /
+// 8.5 / 13.2 against 12.9 / 11.8 / 19.2; random 30k x 8, N = 32 / 128 11.3 / 16.3 against
+// 17.4 / 20.5; random 100k x 8, N = 32 18.8 against 25.8; power-law 100k, N = 32 25.8
+// against 29.4.
+int window_chunk(int nv, int W, int nnz, int most)
+{
+    const long long tiles = (nv + W - 1) / W;
+    const long long workers = (long long)device_sms() * (W == 128 ? 32 : W == 64 ? 64 : 96);
+    const long long per = (W == 128 ? 5 : 8) * (long long)nnz * tiles / (5 * workers);
+    return (int)std::max<long long>(48, std::min<long long>((per + 15) / 16 * 16, most));
+}
+
 // ---------------------------------------------------------------- resolve
 daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int nnz, int nv,
                       const void *B, const void *C, Resolved *out)
@@ -239,7 +255,7 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
                     // 93.3 -> 88.6 us on the power-law matrix), one 64-column
                     // tile at 64 (56.8 -> 53.8 us), wider products (several
                     // tiles in flight) at 128
-                    r.chunk = nv == 128 ? 96 : (nv == 64 ? 64 : 128);
+                    r.chunk = window_chunk(nv, Wt, nnz, nv == 128 ? 96 : (nv == 64 ? 64 : 128));
                 } else {
                     // rings: one wave of chunks over the resident warps (12 per SM)
                     const long long slots = (long long)device_sms() * 12;

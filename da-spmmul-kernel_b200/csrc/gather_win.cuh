@@ -19,6 +19,12 @@ __device__ __forceinline__ void ld_bytes(uint32_t (&w)[NB >= 4 ? NB / 4 : 1], co
     else w[0] = __ldg(reinterpret_cast<const unsigned char *>(p));
 }
 
+// Two choices that give the same bits and differ in what the compiler makes of the
+// window loop; each shape has the faster one (launch_win).
+constexpr int kFormLate = 1;  // a nonzero's value is fetched from its lane with its sum, not
+                              // with its load
+constexpr int kFormLim = 2;   // a window's end is kept, not its length
+
 // The columns of a worker's lane: J vectors of V, vector j at tb + j*G*V.
 template <int G, int V, int J, bool MASK>
 struct WinCols {
@@ -30,7 +36,8 @@ struct WinCols {
 // arrives: piece_arrive for G lanes (`gmask`) and J vectors of V columns per
 // lane.  Templated on the kernel's types so that every kernel has its own
 // copy: ptxas 12.9 crashes (at build time) on one copy shared by two kernels.
-template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK>
+template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK,
+          int FORM>
 static __device__ __noinline__ void piece_arrive_win(const int *__restrict__ rowPtr, int *cnt,
                                                      const float *slots, float *C, int ldc,
                                                      int nv, int chunk, float beta, int row,
@@ -105,8 +112,9 @@ static __device__ __noinline__ void piece_arrive_win(const int *__restrict__ row
 // is stored, the first one's with the window, so no store waits for its load
 // (and all of a window's are prefetched to L2 when the ends are found).  MASK:
 // columns at or past nv are neither loaded (the loads are clamped to the last
-// vector) nor stored.
-template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK>
+// vector) nor stored.  FORM: see kFormLate.
+template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK,
+          int FORM>
 __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
 {
     constexpr int NW = 32 / G;                     // workers per warp
@@ -121,10 +129,7 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
     // slower than unpacking to FP32, so BF16 unpacks)
     constexpr bool PAIR16 =
         std::is_same<TV, fp16>::value && std::is_same<TB, fp16>::value && V >= 2;
-    // Values that need unpacking of B are fetched from their lanes with the sum, not
-    // with the loads: fewer registers while these are in flight (BF16 N = 256 on the
-    // power-law matrix 133 -> 127 us, E4M3 145 -> 129; FP32 161 -> 180, FP16 115 -> 121)
-    constexpr bool LATE = !std::is_same<TB, float>::value && !PAIR16;
+    constexpr bool LATE = (FORM & kFormLate) != 0, LIM = (FORM & kFormLim) != 0;
     const int lane = threadIdx.x & 31, w = lane / G, gl = lane % G;
     const unsigned gmask = GM << (G * w);
     const int tile = blockIdx.y, tiles = gridDim.y;
@@ -263,11 +268,12 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
             cont = false;
         };
         bool sought = false;
+        int lim = ke;  // where this window ends at the latest
         for (; nwin > 0; --nwin) {
-            const int left = ke - wb;  // <= 0: this worker is done
-            int wlen = G;              // (without gaps; a worker's last window may hold fewer)
-            int skip = 0;              // empty rows between this window's and the next one's
+            int wlen = G;  // (without gaps; a worker's last window may hold fewer)
+            int skip = 0;  // empty rows between this window's and the next one's
             if (any_gaps) {
+                const int left = ke - wb;  // <= 0: this worker is done
                 // the first row in sight that is empty, and the window up to it
                 int prev = __shfl_up_sync(kFull, E, 1, G);
                 if (gl == 0) prev = wb;
@@ -301,18 +307,20 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
                     if (seek) r = lo;
                 }
                 if (f > 0 && wlen > 0 && wlen == Ef - wb) skip = max(0, __ffs(live >> f) - 1);
+                lim = wb + wlen;
                 nwin = 1 + (max(0, left - wlen) + G - 1) / G;
 #pragma unroll
                 for (int o = G; o < 32; o <<= 1)
                     nwin = max(nwin, __shfl_xor_sync(kFull, nwin, o));
             }
-            load_win(wb + wlen, cnext, vnext);
+            const int wn = LIM ? min(wb + G, lim) : wb + wlen;
+            load_win(wn, cnext, vnext);
             const int pos = E - 1 - wb;
-            const bool in = r + gl < a.nr && pos >= 0 && pos < min(left, wlen);
+            const bool in = r + gl < a.nr && pos >= 0 &&
+                            (LIM ? E <= wn : pos < min(ke - wb, wlen));
             const unsigned ends =
                 (__reduce_or_sync(kFull, in ? (1u << (pos + G * w)) : 0u) >> (G * w)) & GM;
             prefetch_old(in);
-            wb += wlen;
             // the next window's row ends load while this one is summed
             E = __ldg(a.rowPtr + min(r + __popc(ends) + skip + 1 + gl, a.nr));
             fetch_old(c_row(r), ends != 0);
@@ -347,8 +355,9 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
             }
             if (any_gaps) {
                 r += skip;
-                if (wlen < G && left > wlen) clear();  // it ended with a row: only padding is left
+                if (wn - wb < G && wn < ke) clear();  // it ended with a row: only padding is left
             }
+            wb = wn;
             ccur = cnext;
             vcur = vnext;
         }
@@ -381,11 +390,11 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
             }
         }
         if (head_piece)
-            piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK>(
+            piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK, FORM>(
                 a.rowPtr, a.cnt, a.slots, a.C, a.ldc, a.nv, a.chunk, a.beta, r0, cs.tb, tiles, tile,
                 gmask);
         if (tail)
-            piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK>(
+            piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK, FORM>(
                 a.rowPtr, a.cnt, a.slots, a.C, a.ldc, a.nv, a.chunk, a.beta, s1, cs.tb, tiles, tile,
                 gmask);
         __syncwarp();
@@ -429,7 +438,8 @@ inline void launch_pdl(void (*kernel)(KArgs), dim3 grid, cudaStream_t st, const 
     cudaLaunchKernelEx(&cfg, kernel, a);
 }
 
-template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool MASK>
+template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool MASK,
+          int FORM = 0>
 inline void launch_win_as(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
     constexpr int NW = 32 / G;
@@ -438,9 +448,10 @@ inline void launch_win_as(const Resolved &r, const KArgs &a, cudaStream_t st)
         1, std::min<long long>((groups + 7) / 8, (long long)device_sms() * MINB));
     const dim3 grid(gg, r.tiles);
     if (a.beta == 0.0f)
-        launch_pdl(k_win<G, V, J, U, TV, TB, MINB, false, MASK>, grid, st, a);
+        launch_pdl(k_win<G, V, J, U, TV, TB, MINB, false, MASK, FORM>, grid, st, a);
     else
-        launch_pdl(k_win<G, V, J, U, TV, TB, MINB, true, MASK>, grid, st, a);
+        launch_pdl(k_win<G, V, J, U, TV, TB, MINB, true, MASK,
+                         std::is_same<TB, float>::value ? kFormLim : kFormLate>, grid, st, a);
 }
 
 // B and C aligned for lane loads of V elements (and 32-byte stores from eight
@@ -476,28 +487,32 @@ template <int W, typename TV, typename TB>
 inline void launch_win(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
     constexpr bool f32 = std::is_same<TB, float>::value;
+    constexpr bool f16 = std::is_same<TB, fp16>::value;
+    constexpr bool b2 = sizeof(TB) == 2;
     if constexpr (W == 128) {
         if constexpr (f32) {
             if (win_aligned<TB>(a, 8))
                 return launch_win_as<16, 8, 1, 8, TV, TB, 2, false>(r, a, st);
-        } else if constexpr (sizeof(TB) == 2) {
+        } else if constexpr (b2) {
             if (win_aligned<TB>(a, 8))
-                return launch_win_as<16, 8, 1, 16, TV, TB, 2, false>(r, a, st);
+                return launch_win_as<16, 8, 1, 16, TV, TB, 2, false, kFormLate | kFormLim>(r, a, st);
         } else {
             if (r.tiles == 1 && win_aligned<TB>(a, 8))
-                return launch_win_as<16, 8, 1, 16, TV, TB, 2, false>(r, a, st);
+                return launch_win_as<16, 8, 1, 16, TV, TB, 2, false, kFormLim>(r, a, st);
             if (r.tiles > 1 && win_aligned<TB>(a, 16))
-                return launch_win_as<8, 16, 1, 8, TV, TB, 2, false>(r, a, st);
+                return launch_win_as<8, 16, 1, 8, TV, TB, 2, false, kFormLate>(r, a, st);
         }
         launch_win_as<16, 4, 2, 8, TV, TB, 2, false>(r, a, st);
     } else if constexpr (W == 64) {
-        constexpr int V = sizeof(TB) == 2 ? 4 : 8;
+        constexpr int V = b2 ? 4 : 8;
         if (win_aligned<TB>(a, V))
-            return launch_win_as<64 / V, V, 1, f32 ? 8 : 16, TV, TB, f32 ? 2 : 3, false>(r, a, st);
+            return launch_win_as<64 / V, V, 1, f32 ? 8 : 16, TV, TB, f32 ? 2 : 3, false,
+                                 f16 ? kFormLim : 0>(r, a, st);
         launch_win_as<16, 2, 2, 8, TV, TB, 3, false>(r, a, st);
     } else {
         if (win_aligned<TB>(a, 4))
-            return launch_win_as<8, 4, 1, sizeof(TB) == 2 ? 16 : 8, TV, TB, 3, false>(r, a, st);
+            return launch_win_as<8, 4, 1, b2 ? 16 : 8, TV, TB, 3, false,
+                                 f32 || f16 ? 0 : b2 ? kFormLate : kFormLate | kFormLim>(r, a, st);
         launch_win_as<16, 1, 2, 8, TV, TB, 3, false>(r, a, st);
     }
 }
