@@ -461,10 +461,19 @@ static void launch_transpose_tr(const float *src, long long R, long long Cn, flo
     const unsigned g = (unsigned)std::max<long long>(
         1, std::min<long long>(tiles, (long long)device_sms() * 8));
     const bool vl = Cn % 4 == 0 && aligned(src, 16), vs = R % 4 == 0 && aligned(dst, 16);
-    if (vl && vs) k_transpose<TR, true, true><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
-    else if (vl) k_transpose<TR, true, false><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
-    else if (vs) k_transpose<TR, false, true><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
-    else k_transpose<TR, false, false><<<g, 256, 0, st>>>(src, R, Cn, dst, beta);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(g);
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg,
+                       vl ? (vs ? k_transpose<TR, true, true> : k_transpose<TR, true, false>)
+                          : (vs ? k_transpose<TR, false, true> : k_transpose<TR, false, false>),
+                       src, R, Cn, dst, beta);
 }
 
 static void launch_transpose(const float *src, long long R, long long Cn, float *dst, float beta,

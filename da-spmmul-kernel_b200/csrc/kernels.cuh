@@ -826,6 +826,10 @@ static __global__ void __launch_bounds__(256)
     constexpr int TC = 4096 / TR;
     __shared__ float tile[TR][TC + 1];
     const long long tx = (Cn + TC - 1) / TC, ty = (R + TR - 1) / TR;
+    // a dependent launch: nothing is read or written before the stream's last kernel
+    // has completed
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (long long t = blockIdx.x; t < tx * ty; t += gridDim.x) {
         const long long r0 = (t / tx) * TR, c0 = (t % tx) * TC;
         if constexpr (VL) {
