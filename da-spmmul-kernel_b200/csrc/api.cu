@@ -219,7 +219,9 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
         if (cfg->chunk) r.chunk = cfg->chunk;
         else if (cfg->alg == DASPMM_ALG_COO_VECTOR) r.chunk = std::max(64, 8 * r.S);
         else if (r.cm) r.chunk = 32;
-        else r.chunk = G >= 32 ? 128 : (G >= 16 || (!r.cm && nv > kStreamMaxNv) ? 64 : 32);
+        else if (cfg->alg == DASPMM_ALG_CSR_BALANCED && !r.cm && nv > kStreamMaxNv)
+            r.chunk = G >= 32 ? 128 : 64;
+        else r.chunk = G >= 32 ? 128 : (G >= 16 ? 64 : 32);
         if (r.chunk < 1) return DASPMM_ERR_INVALID;
         if (cfg->alg == DASPMM_ALG_COO_VECTOR && r.chunk % r.S) return DASPMM_ERR_INVALID;
         r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
@@ -765,15 +767,40 @@ static bool spare_workspace(size_t need, size_t most, cudaStream_t st, void **ou
     return cached_workspace(need, st, out) == DASPMM_OK;
 }
 
+// Whether the balanced product is the faster one for a call of algorithm `alg`, by
+// sizes alone: the row lengths are on the device, so a line lies where matrices with
+// even rows (uniform, Poisson), which lose most, break even.  Skewed rows gain more:
+// power-law 262k, row-major N = 128, 681 / 550 / 380 / 438 us -> 83 / 83 / 124 / 124
+// (CSR scalar / CSR vector / COO scalar / COO vector).  us, own kernel -> balanced:
+//   CSR scalar  a warp or less per row, no second launch: row-major uniform 65k x 24,
+//               N = 16 17 -> 23 and 262k x 24, N = 16 45 -> 72, but 262k x 8, N = 64
+//               77 -> 53; column-major random 65k x 2, N = 16 16 -> 35, N = 64 41 -> 30
+//   CSR vector  row-major random 16k x 2, N = 16 9 -> 18, 65k x 2 25 -> 23, 16k x 2, N =
+//               128 25 -> 18; column-major random 4k x 2, N = 16 10 -> 23, N = 64 27 -> 21
+//   COO         under four nonzeros per row the empty rows cut the windows: row-major
+//               random 262k x 2, N = 16 29 -> 44, N = 64 119 -> 62; vector, random 65k x 2,
+//               N = 64 31 -> 35; vector at N <= 8 reads A as fast: 262k x 24, N = 1 62 -> 67,
+//               262k x 8 29 -> 26; vector, random 4k x 24, N = 16 17 -> 19, 16k x 24 27 -> 22
+static bool balanced_pays(int alg, bool cm, int nr, int nnz, int nv)
+{
+    const long long out = (long long)nr * nv;
+    const bool sparse = nnz < 4LL * nr;
+    switch (alg) {
+    case DASPMM_ALG_CSR_SCALAR:
+        return cm ? nv >= 16 && out >= (1 << 22) : nv >= 32 && out >= (1 << 23);
+    case DASPMM_ALG_CSR_VECTOR:
+        return nr >= 65536 || out >= (cm ? 1 << 18 : 1 << 21);
+    case DASPMM_ALG_COO_SCALAR:
+        return cm || nv <= kStreamMaxNv || nv >= 64 || !sparse || out >= (1 << 23);
+    default:
+        if (nv <= kStreamMaxNv) return (cm && nv > 1) || nnz < (1 << 22);
+        return cm || out >= (sparse ? 1 << 23 : 1 << 18) || (!sparse && nv >= 64);
+    }
+}
+
 // A product asked for by one of the reference's four algorithms, none of whose
 // shape the caller chose, runs as the balanced one with the same meaning (sorted
-// rows; COO first makes its row pointer): it is the faster one at every width and
-// layout.  Measured (us, CSR scalar / CSR vector / COO scalar / COO vector -> balanced,
-// COO's conversion included, 262k power-law matrix): 
-//   row-major N = 1   322 / 56 / 79 / 27 -> 16 (COO 22)      4   308 / 88 / 86 / 33 -> 22 (30)
-//            32   359 / 166 / 168 / 135 -> 35 (68)       128  681 / 550 / 380 / 438 -> 83 (124)
-//   col-major  16   876 / 338 / 341 / 168 -> 55 (64)      128 2364 / 2618 / 1470 / 1125 -> 178 (218)
-// (uniform-random rows, row-major, N = 4 / 16 / 32: CSR scalar 18 / 31 / 66 -> 21 / 34 / 38.)
+// rows; COO first makes its row pointer) where that pays.
 // Not (done stays false) where it lacks workspace: column-major operands need copies
 // of B and C, and this library's own block is not grown past kSpareMost for them.
 constexpr size_t kSpareMost = (size_t)2 << 30;
@@ -787,7 +814,8 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
     const bool coo = alg >= DASPMM_ALG_COO_SCALAR;
     // what its own kernels refuse or answer without work stays with them
     if (nr <= 0 || nnz <= 0 || nc <= 0 || !B || !C || !colIdx || !values ||
-        !(coo ? rowIdx : rowPtr))
+        !(coo ? rowIdx : rowPtr) ||
+        !balanced_pays(alg, layout == DASPMM_COL_MAJOR, nr, nnz, nv))
         return DASPMM_OK;
     daspmm_config c{};
     Resolved r;

@@ -80,15 +80,42 @@ def test_not_finite(mats, bad):
                 np.testing.assert_array_equal(C[odd], want[odd])
 
 
+# (rows, average row length, columns): on both sides of each line of the rule that
+# gives a reference algorithm to the balanced product, by algorithm and layout
+_RULE = [(3000, 6, 1), (3000, 6, 16), (3000, 6, 128), (3000, 2, 16), (3000, 2, 64),
+         (70000, 2, 16), (70000, 2, 64), (70000, 6, 1), (70000, 6, 64), (70000, 2, 128)]
+
+
+def _pays(alg, cm, nr, nnz, nv):
+    out, sparse = nr * nv, nnz < 4 * nr
+    if alg == 0:
+        return nv >= 16 and out >= 2**22 if cm else nv >= 32 and out >= 2**23
+    if alg == 1:
+        return nr >= 65536 or out >= (2**18 if cm else 2**21)
+    if alg == 2:
+        return cm or nv <= 8 or nv >= 64 or not sparse or out >= 2**23
+    if nv <= 8:
+        return cm and nv > 1 or nnz < 2**22
+    return cm or out >= (2**23 if sparse else 2**18) or (not sparse and nv >= 64)
+
+
 @pytest.mark.parametrize("layout", [0, 1])
-@pytest.mark.parametrize("nv", [1, 4, 16, 32, 41, 128])
-def test_reference_algorithms_are_the_balanced_product(mats, layout, nv):
-    for name in ("short", "hub", "empty"):
-        A, dA = mats[name]
-        for beta in (0.0, 1.0, 0.5):
-            want = _run(A, dA, 4, layout, nv, beta)[2]
-            for alg in range(4):
-                np.testing.assert_array_equal(_run(A, dA, alg, layout, nv, beta)[2], want)
+@pytest.mark.parametrize("nr,deg,nv", _RULE)
+def test_reference_algorithms(cuda, nr, deg, nv, layout):
+    A = D.gen_random(nr, nr, float(deg), seed=nr + deg)
+    dA = D.DeviceCsr(A)
+    for beta in (0.0, 0.5):
+        want = _run(A, dA, 4, layout, nv, beta)[2]
+        for alg in range(4):
+            B, C0, C = _run(A, dA, alg, layout, nv, beta)
+            _check(A, layout, nv, beta, B, C0, C)
+            if _pays(alg, layout == 1, A.nr, A.nnz, nv):
+                np.testing.assert_array_equal(C, want)
+
+
+def test_coo_scalar_keeps_its_chunk(cuda):
+    for nv, chunk in ((4, 32), (16, 32), (31, 128), (64, 64), (128, 128)):
+        assert D.default_config(2, 0, 1000, 1000, 8000, nv).chunk == chunk
 
 
 def test_inside_a_capture_they_keep_their_own_kernels(mats):
