@@ -116,19 +116,30 @@ static int general_width(int V, int nv)
 
 // Nonzeros per chunk of the window kernel for a tile of W columns: `most`, or fewer
 // where that would leave resident workers without a chunk, but no fewer than 48
-// (shorter chunks cut more rows: power-law 30k rows, N = 128, 23.7 us at 48, 29.5 at 32).
+// (shorter chunks cut more rows: power-law 30k rows, N = 128, 23.7 us at 48, 29.5 at 32),
+// or 32 where rows hold under four nonzeros on average: few are that long, and every empty
+// row cuts a worker's window (random 4k x 2, N = 16 / 128 12.5 / 14.2 us at 32, 14.7 /
+// 16.4 at 48; 65k x 2, N = 64 18.9 against 22.7; but power-law 16k x 8, N = 16 25.9
+// against 19.9).
 // Narrow tiles, whose workers run four to a warp, want a little over one chunk per
 // worker.  us at the chosen chunk against `most`: uniform 4k x 16, N = 32 / 128 / 512 8.6 /
 // 8.5 / 13.2 against 12.9 / 11.8 / 19.2; random 30k x 8, N = 32 / 128 11.3 / 16.3 against
 // 17.4 / 20.5; random 100k x 8, N = 32 18.8 against 25.8; power-law 100k, N = 32 25.8
 // against 29.4.
-int window_chunk(int nv, int W, int nnz, int most)
+int window_chunk(int nv, int W, int nr, int nnz, int most)
 {
+    const int least = nnz < 4LL * nr ? 32 : 48;
     const long long tiles = (nv + W - 1) / W;
     const long long workers = (long long)device_sms() * (W == 128 ? 32 : W == 64 ? 64 : 96);
     const long long per = (W == 128 ? 5 : 8) * (long long)nnz * tiles / (5 * workers);
-    return (int)std::max<long long>(48, std::min<long long>((per + 15) / 16 * 16, most));
+    return (int)std::max<long long>(least, std::min<long long>((per + 15) / 16 * 16, most));
 }
+
+// Rows shorter than this are not cut: half a chunk, or a whole one where chunks are the
+// shortest and the exchange between a row's workers costs more than the longer chunk does
+// (random 4k x 24, N = 16 / 64 / 128 10.4 / 11.5 / 13.2 us against 14.6 / 15.4 / 17.0;
+// 65k x 24, N = 64 at 64 nonzeros 39.5 against 43.2; power-law within 3 %).
+int window_snap(int chunk) { return chunk <= 48 ? chunk : chunk / 2; }
 
 // ---------------------------------------------------------------- resolve
 daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int nnz, int nv,
@@ -257,14 +268,15 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
                     // 93.3 -> 88.6 us on the power-law matrix), one 64-column
                     // tile at 64 (56.8 -> 53.8 us), wider products (several
                     // tiles in flight) at 128
-                    r.chunk = window_chunk(nv, Wt, nnz, nv == 128 ? 96 : (nv == 64 ? 64 : 128));
+                    r.chunk = window_chunk(nv, Wt, nr, nnz, nv == 128 ? 96 : (nv == 64 ? 64 : 128));
                 } else {
                     // rings: one wave of chunks over the resident warps (12 per SM)
                     const long long slots = (long long)device_sms() * 12;
                     r.chunk = (int)std::max<long long>(64, ((long long)nnz + slots - 1) / slots);
                 }
                 r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
-                r.snap = cfg->snap ? std::min(cfg->snap, r.chunk) : r.chunk / 2;
+                r.snap = cfg->snap ? std::min(cfg->snap, r.chunk)
+                                   : r.pipe == 4 ? window_snap(r.chunk) : r.chunk / 2;
             }
         }
     }
@@ -283,6 +295,11 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
         r.general = r.V;
         r.W = general_width(r.V, nv);
         r.block = 256;
+        if (!cfg->chunk) {
+            r.chunk = window_chunk(nv, r.W, nr, nnz, r.chunk);
+            r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
+            r.snap = cfg->snap ? std::min(cfg->snap, r.chunk) : window_snap(r.chunk);
+        }
     }
     const int W = r.general ? r.W : r.L * r.V * r.CF;
     r.tiles = (nv + W - 1) / W;

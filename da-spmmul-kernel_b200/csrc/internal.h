@@ -53,7 +53,8 @@ inline daspmm_config to_config(const Resolved &r)
 extern thread_local int g_last_cuda;
 daspmm_status cuda_fail(cudaError_t e);
 
-int window_chunk(int nv, int W, int nnz, int most);
+int window_chunk(int nv, int W, int nr, int nnz, int most);
+int window_snap(int chunk);
 daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int nnz, int nv,
                       const void *B, const void *C, Resolved *out);
 // What a product asks for, and the least that it can do with.
