@@ -137,7 +137,7 @@ int window_chunk(int nv, int W, int nr, int nnz, int most)
 
 // Rows shorter than this are not cut: half a chunk, or a whole one where chunks are the
 // shortest and the exchange between a row's workers costs more than the longer chunk does
-// (random 4k x 24, N = 16 / 64 / 128 10.4 / 11.5 / 13.2 us against 14.6 / 15.4 / 17.0;
+// (random 4k x 24, N = 64 / 128 11.5 / 13.2 us against 15.4 / 17.0;
 // 65k x 24, N = 64 at 64 nonzeros 39.5 against 43.2; power-law within 3 %).
 int window_snap(int chunk) { return chunk <= 48 ? chunk : chunk / 2; }
 
@@ -296,9 +296,12 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
         r.W = general_width(r.V, nv);
         r.block = 256;
         if (!cfg->chunk) {
-            r.chunk = window_chunk(nv, r.W, nr, nnz, r.chunk);
+            if (nnz < 4LL * nr) r.chunk = window_chunk(nv, r.W, nr, nnz, r.chunk);
             r.nchunks = (int)std::max<long long>(1, ((long long)nnz + r.chunk - 1) / r.chunk);
-            r.snap = cfg->snap ? std::min(cfg->snap, r.chunk) : window_snap(r.chunk);
+            // 64 / 64 against 64 / 32, N = 16: random 4k / 65k x 24 11.7 / 25.8 us
+            // against 14.6 / 30.5, power-law 16k x 8 20.3 against 19.5
+            if (!cfg->snap) r.snap = r.chunk <= 64 ? r.chunk : r.chunk / 2;
+            r.snap = std::min(r.snap, r.chunk);
         }
     }
     const int W = r.general ? r.W : r.L * r.V * r.CF;
@@ -424,7 +427,7 @@ static void launch_all(const Resolved &r, KArgs &a, dim3 grid, dim3 fix_grid, in
                        cudaStream_t st)
 {
     const bool fix = a.nchunks > 1;
-    // the main kernel (pipe 4: the window or walk kernel after k_partition)
+    // the main kernel (pipe 4: the window kernel after k_partition)
     // sits between the optional timer events
     timer_before(st);
     switch (r.alg) {

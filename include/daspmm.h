@@ -81,7 +81,7 @@ typedef struct daspmm_config {
                        row-major product, C transposed back (the default from
                        nv >= 4; A read once for all columns).
                        0 = the library's choice */
-    int l2_window;  /* balanced CSR, row-major window and walk kernels: 0 = off;
+    int l2_window;  /* balanced CSR, row-major window kernels: 0 = off;
                        1..1000 = an L2 access-policy window over B on the main
                        kernel's launch, that many thousandths of its lines
                        marked persisting (the rest streaming).  Has an effect
