@@ -304,6 +304,19 @@ daspmm_status resolve(const daspmm_config *cfg, int layout, int nr, int nc, int 
             r.snap = std::min(r.snap, r.chunk);
         }
     }
+    // Operands off the widest vectors never take more chunks than the aligned ones for
+    // which a workspace is sized (daspmm_workspace_bytes knows no addresses).
+    if (r.pipe == 1 && cfg->alg == DASPMM_ALG_CSR_BALANCED && !r.cm && !r.stream && !cfg->chunk &&
+        (B || C)) {
+        Resolved sized;
+        if (resolve(cfg, layout, nr, nc, nnz, nv, nullptr, nullptr, &sized) == DASPMM_OK &&
+            sized.chunk > r.chunk) {
+            r.chunk = sized.chunk;
+            r.nchunks = sized.nchunks;
+            r.snap = cfg->snap ? std::min(cfg->snap, r.chunk)
+                               : r.general && r.chunk <= 64 ? r.chunk : r.chunk / 2;
+        }
+    }
     const int W = r.general ? r.W : r.L * r.V * r.CF;
     r.tiles = (nv + W - 1) / W;
     if (r.tiles > 65535) return DASPMM_ERR_UNSUPPORTED;
