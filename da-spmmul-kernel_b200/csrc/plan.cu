@@ -25,7 +25,8 @@
 #include <vector>
 
 struct daspmm_plan_s {
-    daspmm::Resolved r;
+    daspmm_config cfg;     // as the caller gave it
+    daspmm::Resolved r;    // of operands aligned to 16 bytes
     int nr, nc, nnz, nv;
     const int *rowPtr, *colIdx;
     const float *values;
@@ -91,6 +92,7 @@ daspmm_status daspmm_plan_create(const daspmm_config *cfg, int nr, int nc, int n
     if (s != DASPMM_OK) return s;
     auto *p = new (std::nothrow) daspmm_plan_s();
     if (!p) return DASPMM_ERR_INVALID;
+    p->cfg = c;
     p->r = r;
     p->nr = nr; p->nc = nc; p->nnz = nnz; p->nv = nv;
     p->rowPtr = rowPtr; p->colIdx = colIdx; p->values = values;
@@ -137,10 +139,15 @@ daspmm_status daspmm_plan_spmm(daspmm_plan p, const float *B, float *C, float be
             return e == cudaSuccess ? DASPMM_OK : daspmm::cuda_fail(e);
         }
     }
-    // the stateless path on the plan's workspace: it rewrites the boundaries
-    // and the queue heads, so the next planned call refreshes them
+    // the stateless path on the plan's workspace, with the vectors that these addresses
+    // allow (p->r's may be wider); it rewrites the boundaries and the queue heads, so the
+    // next planned call refreshes them
+    daspmm::Resolved r;
+    const daspmm_status s = daspmm::resolve(&p->cfg, DASPMM_ROW_MAJOR, p->nr, p->nc, p->nnz, p->nv,
+                                            B, C, &r);
+    if (s != DASPMM_OK) return s;
     p->fresh = false;
-    return daspmm::run_resolved(p->r, DASPMM_ROW_MAJOR, p->nr, p->nc, p->nnz, p->nv, p->rowPtr,
+    return daspmm::run_resolved(r, DASPMM_ROW_MAJOR, p->nr, p->nc, p->nnz, p->nv, p->rowPtr,
                                 nullptr, p->colIdx, p->values, B, C, beta, p->ws, p->ws_bytes,
                                 st);
 }
