@@ -739,25 +739,49 @@ struct WsKey {
         return tag < o.tag;
     }
 };
-static std::recursive_mutex g_ws_mu;
-std::recursive_mutex &workspace_mutex() { return g_ws_mu; }
-static std::map<WsKey, std::pair<void *, size_t>> g_ws;
+struct WsBlock {
+    std::recursive_mutex mu;  // held from the request until the caller's work is queued
+    void *p = nullptr;
+    size_t bytes = 0;
+};
+static std::mutex g_ws_mu;  // the map alone: a block that grows holds up its own stream only
+static std::map<WsKey, WsBlock> g_ws;  // (never erased: references stay good)
+
+static WsBlock *block_of(cudaStream_t st, int tag)
+{
+    int dev = 0;
+    const cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) {
+        cuda_fail(e);
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lk(g_ws_mu);
+    return &g_ws[WsKey{dev, (void *)st, tag}];
+}
+
+static WorkspaceLock hold_block(cudaStream_t st, int tag)
+{
+    WsBlock *b = block_of(st, tag);
+    return b ? WorkspaceLock(b->mu) : WorkspaceLock();
+}
+
+WorkspaceLock hold_workspace(cudaStream_t st) { return hold_block(st, 0); }
 
 static daspmm_status cached_block(size_t need, cudaStream_t st, int tag, void **out)
 {
     *out = nullptr;
     if (need == 0) return DASPMM_OK;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return cuda_fail(e);
-    std::lock_guard<std::recursive_mutex> lk(g_ws_mu);
-    auto &slot = g_ws[WsKey{dev, (void *)st, tag}];
-    if (slot.second < need) {
-        if (slot.first) {
+    WsBlock *b = block_of(st, tag);
+    if (!b) return DASPMM_ERR_CUDA;
+    std::lock_guard<std::recursive_mutex> lk(b->mu);
+    if (b->bytes < need) {
+        cudaError_t e;
+        if (b->p) {
             e = cudaStreamSynchronize(st);
             if (e != cudaSuccess) return cuda_fail(e);
-            cudaFree(slot.first);
-            slot = {nullptr, 0};
+            cudaFree(b->p);
+            b->p = nullptr;
+            b->bytes = 0;
         }
         void *p = nullptr;
         const size_t bytes = std::max(need, (size_t)1 << 20);
@@ -767,9 +791,10 @@ static daspmm_status cached_block(size_t need, cudaStream_t st, int tag, void **
             g_last_cuda = (int)e;
             return DASPMM_ERR_NOMEM;
         }
-        slot = {p, bytes};
+        b->p = p;
+        b->bytes = bytes;
     }
-    *out = slot.first;
+    *out = b->p;
     return DASPMM_OK;
 }
 
@@ -795,8 +820,8 @@ static bool spare_workspace(size_t need, size_t most, cudaStream_t st, void **ou
         cudaGetLastError();
         return false;
     }
-    auto it = g_ws.find(WsKey{dev, (void *)st, 0});
-    if ((it == g_ws.end() || it->second.second < need) && need > most) return false;
+    const WsBlock *b = block_of(st, 0);
+    if (!b || (b->bytes < need && need > most)) return false;
     return cached_workspace(need, st, out) == DASPMM_OK;
 }
 
@@ -858,7 +883,7 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
     const size_t rows = coo ? align256(sizeof(int) * ((size_t)nr + 1)) : 0;
     const size_t need = workspace_bytes(r, nv);
-    std::lock_guard<std::recursive_mutex> hold(g_ws_mu);
+    const WorkspaceLock hold = hold_workspace(st);
     void *ws = nullptr;
     if (!spare_workspace(rows + need, kSpareMost, st, &ws)) return DASPMM_OK;
     char *own = (char *)ws + rows;
@@ -932,9 +957,9 @@ daspmm_status daspmm_spmm_ex(const daspmm_config *cfg, int layout, int nr, int n
     daspmm_status s = resolve(cfg, layout, nr, nc, nnz, nv, B, C, &r);
     if (s != DASPMM_OK) return s;
     cudaStream_t st = (cudaStream_t)stream;
-    std::unique_lock<std::recursive_mutex> hold(workspace_mutex(), std::defer_lock);
+    WorkspaceLock hold;
     if (!workspace) {
-        hold.lock();
+        hold = hold_workspace(st);
         const size_t need = workspace_bytes(r, nv);
         s = cached_workspace(need, st, &workspace);
         if (s != DASPMM_OK) return s;
@@ -1018,8 +1043,10 @@ daspmm_status daspmm_ownership(int alg, int nr, int nnz, const int *rowPtr, cons
     a.nchunks = daspmm_num_chunks(nnz, chunk);
     a.own = owner;
     void *meta = nullptr;
+    WorkspaceLock hold;
     if (alg == DASPMM_ALG_CSR_BALANCED) {
         if (!rowPtr) return DASPMM_ERR_INVALID;
+        hold = hold_workspace(st);
         daspmm_status s = cached_workspace(sizeof(int2) * ((size_t)a.nchunks + 1), st, &meta);
         if (s != DASPMM_OK) return s;
         s = daspmm_partition(nr, nnz, rowPtr, chunk, snap, (int *)meta, stream);
@@ -1177,6 +1204,7 @@ static daspmm_status spmm_host_impl(const daspmm_config *cfg, int layout, int nr
     const size_t b_ws = workspace_bytes(r, nv);
     const size_t total = b_rp + b_ri + b_ci + b_va + b_B + b_C + b_ws;
     void *blk = nullptr;
+    WorkspaceLock hold = hold_block(st, 1);
     s = cached_host_staging(total, st, &blk);
     if (s != DASPMM_OK) return s;
     char *p = (char *)blk;
@@ -1203,6 +1231,7 @@ static daspmm_status spmm_host_impl(const daspmm_config *cfg, int layout, int nr
                      b_ws, st);
     if (s != DASPMM_OK) return s;
     e = cudaMemcpyAsync(C, d_C, sizeof(float) * (size_t)nr * nv, cudaMemcpyDeviceToHost, st);
+    if (hold) hold.unlock();  // everything is queued
     if (e == cudaSuccess && sync) e = cudaStreamSynchronize(st);
     return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
 }

@@ -76,10 +76,12 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
 // zeroed queue state of the balanced split).
 void carve_and_partition(const Resolved &r, int nr, int nnz, int nv, const int *rowPtr, void *ws,
                          size_t ws_bytes, cudaStream_t st);
-// The library's workspace of (device, stream).  A caller holds the lock from before
+// The library's workspace of (device, stream).  A caller holds its lock from before
 // it asks until its kernels are queued: another thread's larger request waits for
-// the stream before it frees the block.
-std::recursive_mutex &workspace_mutex();
+// the stream before it frees the block.  One lock per (device, stream): a call whose
+// block grows does not hold up those of other streams.
+using WorkspaceLock = std::unique_lock<std::recursive_mutex>;
+WorkspaceLock hold_workspace(cudaStream_t st);
 daspmm_status cached_workspace(size_t need, cudaStream_t st, void **out);
 // A planned FP32 row-major balanced-CSR product (plan.cu), beta == 0: the
 // window kernel alone, over a workspace whose chunk boundaries k_partition

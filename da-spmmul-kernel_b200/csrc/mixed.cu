@@ -9,7 +9,6 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <mutex>
 
 namespace daspmm {
 
@@ -310,9 +309,9 @@ daspmm_status daspmm_spmm_mixed(const daspmm_config *cfg_in, int layout, int nr,
     if (nr == 0) return DASPMM_OK;
     if (!B || !C || !rowPtr || (nnz > 0 && (!colIdx || !values))) return DASPMM_ERR_INVALID;
     cudaStream_t st = (cudaStream_t)stream;
-    std::unique_lock<std::recursive_mutex> hold(workspace_mutex(), std::defer_lock);
+    WorkspaceLock hold;
     if (!workspace) {
-        hold.lock();
+        hold = hold_workspace(st);
         const size_t need = workspace_bytes(r, nv);
         s = cached_workspace(need, st, &workspace);
         if (s != DASPMM_OK) return s;

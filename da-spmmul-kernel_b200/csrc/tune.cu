@@ -72,6 +72,7 @@ daspmm_status fingerprint(int layout, int nr, int nnz, int nv, int dtype, const 
         unsigned long long *d_hist = nullptr;
         int *d_max = nullptr;
         void *blk = nullptr;
+        const WorkspaceLock hold = hold_workspace(st);
         daspmm_status s = cached_workspace(33 * sizeof(unsigned long long) + 256, st, &blk);
         if (s != DASPMM_OK) return s;
         d_hist = (unsigned long long *)blk;
