@@ -14,6 +14,7 @@
 #include "gather_stream.cuh"
 #include "internal.h"
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -82,6 +83,39 @@ daspmm_status cuda_fail(cudaError_t e)
 {
     g_last_cuda = (int)e;
     return DASPMM_ERR_CUDA;
+}
+
+// The two driver functions are reached through the runtime, so the library does not
+// link libcuda itself.
+unsigned long long current_context_id()
+{
+    using GetCurrent = CUresult (*)(CUcontext *);
+    using GetId = CUresult (*)(CUcontext, unsigned long long *);
+    struct Driver {
+        GetCurrent current = nullptr;
+        GetId id = nullptr;
+        Driver()
+        {
+            void *f1 = nullptr, *f2 = nullptr;
+            cudaDriverEntryPointQueryResult q1 = cudaDriverEntryPointSymbolNotFound, q2 = q1;
+            if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f1, cudaEnableDefault, &q1) ==
+                    cudaSuccess &&
+                q1 == cudaDriverEntryPointSuccess &&
+                cudaGetDriverEntryPoint("cuCtxGetId", &f2, cudaEnableDefault, &q2) ==
+                    cudaSuccess &&
+                q2 == cudaDriverEntryPointSuccess) {
+                current = reinterpret_cast<GetCurrent>(f1);
+                id = reinterpret_cast<GetId>(f2);
+            }
+        }
+    };
+    static const Driver drv;
+    CUcontext ctx = nullptr;
+    unsigned long long id = 0;
+    if (!drv.current || drv.current(&ctx) != CUDA_SUCCESS || !ctx ||
+        drv.id(ctx, &id) != CUDA_SUCCESS)
+        return 0;
+    return id;
 }
 
 static int pow2ceil(int x)
@@ -808,22 +842,91 @@ daspmm_status cached_host_staging(size_t need, cudaStream_t st, void **out)
     return cached_block(need, st, 1, out);
 }
 
-// A block of the cached workspace without an error where there is none: not when it
-// would have to grow beyond `most`, without memory, or inside a stream capture (a
-// graph would keep the address of a block that a later call may replace).
-static bool spare_workspace(size_t need, size_t most, cudaStream_t st, void **out)
+// ---------------------------------------------------------------- scratch of routed calls
+// The scratch of a call that is routed to the balanced product (through_balanced) and
+// needed none by itself: taken from the stream's own order out of a pool of this library,
+// and given back in it when the call's kernels are queued.  So it is no part of the
+// workspace above (whose address a captured graph may hold), threads and streams share
+// nothing, and what is idle beyond kScratchKeep returns to the device at the next
+// synchronisation (the rest with daspmm_scratch_trim).
+constexpr size_t kScratchMost = (size_t)2 << 30;    // of one call
+constexpr size_t kScratchKeep = (size_t)512 << 20;  // idle, per device
+
+static cudaMemPool_t scratch_pool(bool make)
 {
+    struct Pool {
+        unsigned long long ctx;
+        cudaMemPool_t pool;
+    };
+    static std::mutex mu;
+    static std::map<int, Pool> pools;
     int dev = 0;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaStreamIsCapturing(st, &cap) != cudaSuccess ||
-        cap != cudaStreamCaptureStatusNone) {
+    if (cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return nullptr;
     }
-    const WsBlock *b = block_of(st, 0);
-    if (!b || (b->bytes < need && need > most)) return false;
-    return cached_workspace(need, st, out) == DASPMM_OK;
+    std::lock_guard<std::mutex> lk(mu);
+    const unsigned long long ctx = current_context_id();
+    auto it = pools.find(dev);
+    if (it != pools.end() && it->second.ctx == ctx) return it->second.pool;
+    // none yet, or that of a context which cudaDeviceReset has ended
+    if (!make || ctx == 0) return nullptr;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    unsigned long long keep = kScratchKeep;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        pool = nullptr;  // not asked again: such calls keep their own kernels
+    }
+    pools[dev] = Pool{ctx, pool};
+    return pool;
 }
+
+// Allocation is not part of what a thread may be capturing on another stream.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+class Scratch {
+    cudaStream_t st;
+    void *p = nullptr;
+
+public:
+    explicit Scratch(cudaStream_t s) : st(s) {}
+    Scratch(const Scratch &) = delete;
+    ~Scratch()
+    {
+        if (!p) return;
+        OutsideCapture out;
+        cudaFreeAsync(p, st);
+    }
+    // Null, without an error, where there is none: more than kScratchMost, no memory, or
+    // inside a stream capture.
+    void *take(size_t need)
+    {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (need > kScratchMost) return nullptr;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        if (cap != cudaStreamCaptureStatusNone) return nullptr;
+        OutsideCapture out;
+        cudaMemPool_t pool = scratch_pool(true);
+        if (!pool) return nullptr;
+        if (cudaMallocFromPoolAsync(&p, need, pool, st) != cudaSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return p;
+    }
+};
 
 // Whether the balanced product is the faster one for a call of algorithm `alg`, by
 // sizes alone: the row lengths are on the device, so a line lies where matrices with
@@ -859,9 +962,7 @@ static bool balanced_pays(int alg, bool cm, int nr, int nnz, int nv)
 // A product asked for by one of the reference's four algorithms, none of whose
 // shape the caller chose, runs as the balanced one with the same meaning (sorted
 // rows; COO first makes its row pointer) where that pays.
-// Not (done stays false) where it lacks workspace: column-major operands need copies
-// of B and C, and this library's own block is not grown past kSpareMost for them.
-constexpr size_t kSpareMost = (size_t)2 << 30;
+// Not (done stays false) where there is no scratch for it.
 static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int nnz, int nv,
                                       const int *rowPtr, const int *rowIdx, const int *colIdx,
                                       const float *values, const float *B, float *C, float beta,
@@ -883,9 +984,9 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
     const size_t rows = coo ? align256(sizeof(int) * ((size_t)nr + 1)) : 0;
     const size_t need = workspace_bytes(r, nv);
-    const WorkspaceLock hold = hold_workspace(st);
-    void *ws = nullptr;
-    if (!spare_workspace(rows + need, kSpareMost, st, &ws)) return DASPMM_OK;
+    Scratch scratch(st);
+    void *ws = scratch.take(rows + need);
+    if (!ws) return DASPMM_OK;
     char *own = (char *)ws + rows;
     if (coo) {
         // where the row-major product's boundaries will lie (k_stream keeps none)
@@ -1072,6 +1173,14 @@ daspmm_status daspmm_coo_to_csr(int nr, int nnz, const int *rowIdx, int *rowPtr,
     k_coo_to_csr<<<g, 256, 0, (cudaStream_t)stream>>>(nr, nnz, rowIdx, rowPtr);
     count_launches(1);
     cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
+}
+
+daspmm_status daspmm_scratch_trim(size_t keep)
+{
+    cudaMemPool_t pool = scratch_pool(false);
+    if (!pool) return DASPMM_OK;
+    const cudaError_t e = cudaMemPoolTrimTo(pool, keep);
     return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
 }
 

@@ -52,6 +52,10 @@ inline daspmm_config to_config(const Resolved &r)
 
 extern thread_local int g_last_cuda;
 daspmm_status cuda_fail(cudaError_t e);
+// The id of the current device's current context (0 when it cannot be read, or before
+// this thread's first runtime call); cudaDeviceReset ends a context, and the next one has
+// another id.
+unsigned long long current_context_id();
 
 int window_chunk(int nv, int W, int nr, int nnz, int most);
 int window_snap(int chunk);

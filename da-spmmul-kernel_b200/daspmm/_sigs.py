@@ -59,6 +59,7 @@ class MtxHeader(ctypes.Structure):
 
 def apply(lib, Config):
     sig = {
+        "daspmm_scratch_trim": (_I, [ctypes.c_size_t]),
         "daspmm_batch_create": (_I, [ctypes.POINTER(Instance), _I, ctypes.POINTER(Config),
                                      ctypes.POINTER(_VP), _VP]),
         "daspmm_batch_run": (_I, [_VP, _VP]),

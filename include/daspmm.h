@@ -92,9 +92,14 @@ typedef struct daspmm_config {
 /* ---- FP32 SpMM ---------------------------------------------------------
  * C = A*B + beta*C.  beta == 0 never reads C.  For the COO algorithms a beta
  * other than 1 first scales all of C (rows without nonzeros included).
- * Uses a workspace the library keeps per (device, stream); the call that first
- * needs a larger one synchronises the stream and allocates (so it must not be
- * the first call inside a stream capture).
+ * Balanced CSR and the COO kernels use a workspace the library keeps per (device,
+ * stream); the call that first needs a larger one synchronises the stream and
+ * allocates (so it must not be the first call inside a stream capture).
+ * The algorithms 0..3 run as the balanced product where that is faster.  Their
+ * scratch for it (column-major: copies of B and C) comes from a pool of the
+ * library in the stream's order; a call that gets none, because it would need
+ * more than 2 GiB, there is no memory, or its stream is being captured, runs its
+ * own kernels.  See daspmm_scratch_trim.
  * Replaces: cudaSpmm<kBlockSize,kWarpSize>(alg, layout, nr, nc, nnz, nv,
  * rowPtr, rowIdx, colIdx, values, dnInput, dnOutput) (spmvspmm.h:53-199),
  * which has beta fixed by the algorithm. */
@@ -112,6 +117,11 @@ daspmm_status daspmm_spmm_ex(const daspmm_config *cfg, int layout, int nr, int n
                              const int *colIdx, const float *values, const float *B,
                              float *C, float beta, void *workspace, size_t ws_bytes,
                              void *stream);
+
+/* Gives the idle memory of the current device's scratch pool back to the device, down
+ * to `keep` bytes (at most 512 MiB stay there otherwise).  No counterpart in the
+ * reference, which allocates nothing. */
+daspmm_status daspmm_scratch_trim(size_t keep);
 
 /* Workspace bytes daspmm_spmm_ex needs for this configuration and shape
  * (pipe 5 holds row-major copies of B and C, so nc matters). */
