@@ -951,6 +951,8 @@ static bool balanced_pays(int alg, bool cm, int nr, int nnz, int nv)
         return cm ? nv >= 16 && out >= (1 << 22) : nv >= 32 && out >= (1 << 23);
     case DASPMM_ALG_CSR_VECTOR:
         return nr >= 65536 || out >= (cm ? 1 << 18 : 1 << 21);
+    case DASPMM_ALG_AUTO:
+        return true;
     case DASPMM_ALG_COO_SCALAR:
         return cm || nv <= kStreamMaxNv || nv >= 64 || !sparse || out >= (1 << 23);
     default:
@@ -960,7 +962,8 @@ static bool balanced_pays(int alg, bool cm, int nr, int nnz, int nv)
 }
 
 // A product asked for by one of the reference's four algorithms, none of whose
-// shape the caller chose, runs as the balanced one with the same meaning (sorted
+// shape the caller chose, or by AUTO where nothing has been tuned and the rule of
+// thumb is CSR scalar, runs as the balanced one with the same meaning (sorted
 // rows; COO first makes its row pointer) where that pays.
 // Not (done stays false) where there is no scratch for it.
 static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int nnz, int nv,
@@ -969,8 +972,7 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
                                       cudaStream_t st, bool *done)
 {
     *done = false;
-    if (alg < DASPMM_ALG_CSR_SCALAR || alg > DASPMM_ALG_COO_VECTOR) return DASPMM_OK;
-    const bool coo = alg >= DASPMM_ALG_COO_SCALAR;
+    const bool coo = alg == DASPMM_ALG_COO_SCALAR || alg == DASPMM_ALG_COO_VECTOR;
     // what its own kernels refuse or answer without work stays with them
     if (nr <= 0 || nnz <= 0 || nc <= 0 || !B || !C || !colIdx || !values ||
         !(coo ? rowIdx : rowPtr) ||
@@ -978,7 +980,7 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
         return DASPMM_OK;
     daspmm_config c{};
     Resolved r;
-    c.alg = alg;
+    c.alg = alg == DASPMM_ALG_AUTO ? DASPMM_ALG_CSR_SCALAR : alg;
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
     c.alg = DASPMM_ALG_CSR_BALANCED;
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
@@ -1076,11 +1078,18 @@ daspmm_status daspmm_spmm(int alg, int layout, int nr, int nc, int nnz, int nv,
                           void *stream)
 {
     daspmm_config c{};
+    bool route = alg >= DASPMM_ALG_CSR_SCALAR && alg <= DASPMM_ALG_COO_VECTOR;
     if (alg == DASPMM_ALG_AUTO) {
-        daspmm_status s = tuned_config(layout, nr, nc, nnz, nv, &c);
+        bool tuned = false;
+        daspmm_status s = tuned_config(layout, nr, nc, nnz, nv, &c, &tuned);
+        Resolved r;
+        if (s == DASPMM_OK) s = resolve(&c, layout, nr, nc, nnz, nv, B, C, &r);
         if (s != DASPMM_OK) return s;
+        route = !tuned && c.alg == DASPMM_ALG_CSR_SCALAR;
     } else {
         c.alg = alg;
+    }
+    if (route) {
         bool done = false;
         const daspmm_status s = through_balanced(alg, layout, nr, nc, nnz, nv, rowPtr, rowIdx,
                                                  colIdx, values, B, C, beta, (cudaStream_t)stream,

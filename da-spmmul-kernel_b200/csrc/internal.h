@@ -176,8 +176,9 @@ daspmm_status batch_kernel_async(int val_fmt, int b_fmt, int wmode, bool grp,
                                  const BatchInst *d_inst, const BatchItem *d_items,
                                  long long nitems, unsigned long long *d_head, cudaStream_t st);
 
-// Autotuner (tune.cu): the cached best configuration for a shape, or the
+// Autotuner (tune.cu): the cached best configuration for a shape (*tuned), or the
 // library's rule-of-thumb choice when nothing has been measured yet.
-daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_config *out);
+daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_config *out,
+                           bool *tuned = nullptr);
 
 }  // namespace daspmm

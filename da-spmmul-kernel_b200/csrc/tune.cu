@@ -181,7 +181,8 @@ float time_config(const daspmm_config &c, int layout, int nr, int nc, int nnz, i
 
 }  // namespace
 
-daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_config *out)
+daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_config *out,
+                           bool *tuned)
 {
     (void)nc;
     {
@@ -189,14 +190,17 @@ daspmm_status tuned_config(int layout, int nr, int nc, int nnz, int nv, daspmm_c
         auto it = g_cache.find(Key{layout, nv, nr, nnz});
         if (it != g_cache.end()) {
             *out = it->second.cfg;
+            if (tuned) *tuned = true;
             return DASPMM_OK;
         }
     }
-    // Untuned shapes: the balanced split, the fastest at every width and layout
-    // that was measured (k_stream up to 16 columns, the window kernel above,
-    // through transposes for column-major operands).
+    if (tuned) *tuned = false;
+    // Untuned shapes: the balanced split for wide dense operands (B rows of >= 128
+    // bytes), otherwise the row-balanced scalar kernel, which needs no workspace
+    // (daspmm_spmm runs such a call as the balanced product where it has scratch).
     daspmm_config c{};
-    c.alg = DASPMM_ALG_CSR_BALANCED;
+    c.alg = (layout == DASPMM_ROW_MAJOR && nv >= 32) ? DASPMM_ALG_CSR_BALANCED
+                                                      : DASPMM_ALG_CSR_SCALAR;
     Resolved r;
     daspmm_status s = resolve(&c, layout, nr, nc, nnz, nv, nullptr, nullptr, &r);
     if (s != DASPMM_OK) return s;

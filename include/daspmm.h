@@ -95,7 +95,8 @@ typedef struct daspmm_config {
  * Balanced CSR and the COO kernels use a workspace the library keeps per (device,
  * stream); the call that first needs a larger one synchronises the stream and
  * allocates (so it must not be the first call inside a stream capture).
- * The algorithms 0..3 run as the balanced product where that is faster.  Their
+ * The algorithms 0..3 run as the balanced product where that is faster, and so does
+ * AUTO where nothing has been tuned and its configuration is CSR scalar.  Their
  * scratch for it (column-major: copies of B and C) comes from a pool of the
  * library in the stream's order; a call that gets none, because it would need
  * more than 2 GiB, there is no memory, or its stream is being captured, runs its
