@@ -520,10 +520,10 @@ static daspmm_status dispatch(const Resolved &r, KArgs &a, dim3 grid, dim3 fix_g
     return DASPMM_ERR_UNSUPPORTED;
 }
 
-// dst (Cn x R, row-major) = transpose of src (R x Cn, row-major) + beta * dst.
-template <int TR>
+// dst (Cn x R, row-major) = transpose of src (R x Cn, row-major) + beta * dst.  KEEP: the columns of dst whose row of the matrix is empty are left as they are.
+template <int TR, bool KEEP>
 static void launch_transpose_tr(const float *src, long long R, long long Cn, float *dst,
-                                float beta, cudaStream_t st)
+                                float beta, const int *rowPtr, cudaStream_t st)
 {
     constexpr int TC = 4096 / TR;
     const long long tiles = ((R + TR - 1) / TR) * ((Cn + TC - 1) / TC);
@@ -540,19 +540,21 @@ static void launch_transpose_tr(const float *src, long long R, long long Cn, flo
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg,
-                       vl ? (vs ? k_transpose<TR, true, true> : k_transpose<TR, true, false>)
-                          : (vs ? k_transpose<TR, false, true> : k_transpose<TR, false, false>),
-                       src, R, Cn, dst, beta);
+                       vl ? (vs ? k_transpose<TR, true, true, KEEP> : k_transpose<TR, true, false, KEEP>)
+                          : (vs ? k_transpose<TR, false, true, KEEP>
+                                : k_transpose<TR, false, false, KEEP>),
+                       src, R, Cn, dst, beta, rowPtr);
 }
 
+template <bool KEEP = false>
 static void launch_transpose(const float *src, long long R, long long Cn, float *dst, float beta,
-                             cudaStream_t st)
+                             cudaStream_t st, const int *rowPtr = nullptr)
 {
-    if (R <= 16) launch_transpose_tr<16>(src, R, Cn, dst, beta, st);
-    else if (R <= 32) launch_transpose_tr<32>(src, R, Cn, dst, beta, st);
-    else if (Cn <= 16) launch_transpose_tr<256>(src, R, Cn, dst, beta, st);
-    else if (Cn <= 32) launch_transpose_tr<128>(src, R, Cn, dst, beta, st);
-    else launch_transpose_tr<64>(src, R, Cn, dst, beta, st);
+    if (R <= 16) launch_transpose_tr<16, KEEP>(src, R, Cn, dst, beta, rowPtr, st);
+    else if (R <= 32) launch_transpose_tr<32, KEEP>(src, R, Cn, dst, beta, rowPtr, st);
+    else if (Cn <= 16) launch_transpose_tr<256, KEEP>(src, R, Cn, dst, beta, rowPtr, st);
+    else if (Cn <= 32) launch_transpose_tr<128, KEEP>(src, R, Cn, dst, beta, rowPtr, st);
+    else launch_transpose_tr<64, KEEP>(src, R, Cn, dst, beta, rowPtr, st);
     count_launches(1);
 }
 
@@ -623,7 +625,9 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
         s = run_resolved(in, DASPMM_ROW_MAJOR, nr, nc, nnz, nv, rowPtr, rowIdx, colIdx, values,
                          Brm, Crm, 0.0f, iws, workspace_bytes(in, nv), st);
         if (s != DASPMM_OK) return s;
-        launch_transpose(Crm, nr, nv, C, beta, st);  // C = transpose + beta * C
+        // C = transpose + beta * C; with beta == 1 rows without nonzeros are C's already
+        if (beta == 1.0f) launch_transpose<true>(Crm, nr, nv, C, beta, st, rowPtr);
+        else launch_transpose(Crm, nr, nv, C, beta, st);
         const cudaError_t e = cudaGetLastError();
         return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
     }
@@ -757,7 +761,7 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, k_partition, nr, nnz, rowPtr, (int)r.chunk, (int)r.snap,
                        (int)r.nchunks, const_cast<int2 *>(a.meta), a.cnt, (int)r.tiles, a.head,
-                       a.emap, rows_beta ? a.C : (float *)nullptr, a.nv, a.beta);
+                       a.emap, rows_beta && a.beta != 1.0f ? a.C : (float *)nullptr, a.nv, a.beta);
     count_launches(1);
 }
 

@@ -56,8 +56,10 @@ __device__ __forceinline__ int row_of(const int *__restrict__ rowPtr, int nr, in
 }
 
 // NV: nv where it is known at compile time, else 0.  V floats per load of B (nv % V
-// == 0, B aligned to them).  CMB / CMC: B / C column-major (B only with V == 1).
-template <int NV, int V, bool CMB, bool CMC>
+// == 0, B aligned to them).  CMB / CMC: B / C column-major (B only with V == 1).  ONE: beta
+// is 1, so a row without nonzeros is C's already and not touched (a form of its own: the
+// check in one form for all cost 1 % at one and eight columns).
+template <int NV, int V, bool CMB, bool CMC, bool ONE>
 __global__ void __launch_bounds__(256) k_stream(const KArgs a)
 {
     extern __shared__ __align__(16) float stream_mem[];
@@ -149,6 +151,7 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     // (row, VC columns) of thread t, then every 256 further: row-major, columns next to
     // each other, so a warp stores whole lines; column-major, rows.
     constexpr int VC = CMC ? 1 : V;
+    constexpr int least = ONE ? 1 : 0;  // nonzeros of the rows that are written
     const int fast = CMC ? max(rows, 1) : nv / VC;
     int lo = t % fast, hi = t / fast;
     const int dlo = 256 % fast, dhi = 256 / fast;
@@ -156,8 +159,9 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
         const int row = r0 + (CMC ? lo : hi), k = CMC ? hi : lo * VC;
         if (CMC && lo >= rows) continue;
         const int p0 = max(__ldg(a.rowPtr + row), k0), p1 = min(__ldg(a.rowPtr + row + 1), k1);
-        if (p1 - p0 >= kStreamLong) {
-            if (k == 0) {
+        const int len = p1 - p0;
+        if ((unsigned)(len - least) >= (unsigned)(kStreamLong - least)) {  // long, or not written
+            if (k == 0 && len > 0) {
                 const int q = atomicAdd(&nlong, 1);
                 if (q < 64) longs[q] = row;  // (a chunk holds fewer)
             }
@@ -262,7 +266,8 @@ inline void launch_stream_as(const KArgs &a, cudaStream_t st)
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_stream<NV, V, CMB, CMC>, a);
+    cudaLaunchKernelEx(&cfg, a.beta == 1.0f ? k_stream<NV, V, CMB, CMC, true>
+                                            : k_stream<NV, V, CMB, CMC, false>, a);
     if (a.nchunks > 1) {
         cfg.gridDim = dim3((unsigned)((a.nchunks - 1 + 7) / 8));
         cfg.dynamicSmemBytes = 0;

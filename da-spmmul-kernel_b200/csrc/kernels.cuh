@@ -551,8 +551,8 @@ __global__ void __launch_bounds__(256) k_fix_coo(const KArgs a)
 // threshold that straddle chunk boundaries.
 // ======================================================================
 // The window kernel leaves rows without nonzeros to this pass: with C they are
-// finished here (C = beta*C, nv columns, the warp together), with emap their
-// bitmap is kept.
+// finished here (C = beta*C, nv columns, the warp together; beta == 1 needs no pass
+// and gets no C, so such rows are not touched), with emap their bitmap is kept.
 static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowPtr,
                             int chunk, int snap, int nchunks, int2 *meta, int *cnt, int tiles,
                             unsigned int *head, unsigned int *emap, float *C, int nv, float beta)
@@ -809,7 +809,9 @@ __global__ void __launch_bounds__(256) k_fix_bal(const KArgs a)
 }
 
 // dst (Cn x R) = transpose of src (R x Cn) + beta * dst, both row-major; beta ==
-// 0 never reads dst.  Bound by memory (each element read and written once), so
+// 0 never reads dst.  KEEP: rowPtr is a row pointer over the R rows; the columns of dst
+// whose row is empty are neither read nor written (another stream may be adding to
+// them).  Bound by memory (each element read and written once), so
 // what counts is bytes in flight: a CTA moves a tile of 4096 elements, 64 bytes
 // per thread in flight before the one barrier, eight CTAs per SM, with 16-byte
 // accesses on either side where sizes and addresses allow (VL: Cn % 4 == 0 and
@@ -818,13 +820,14 @@ __global__ void __launch_bounds__(256) k_fix_bal(const KArgs a)
 // the tile lies outside it.  The odd pitch keeps shared-memory conflicts at two
 // ways.  128 x 262,144: 98 us with 32 x 32 tiles of single accesses, 42 us here
 // (6.4 TB/s); back 95 us, now 40.
-template <int TR, bool VL, bool VS>
+template <int TR, bool VL, bool VS, bool KEEP>
 static __global__ void __launch_bounds__(256)
     k_transpose(const float *__restrict__ src, long long R, long long Cn,
-                float *__restrict__ dst, float beta)
+                float *__restrict__ dst, float beta, const int *__restrict__ rowPtr)
 {
     constexpr int TC = 4096 / TR;
     __shared__ float tile[TR][TC + 1];
+    __shared__ bool keep[KEEP ? TR : 1];
     const long long tx = (Cn + TC - 1) / TC, ty = (R + TR - 1) / TR;
     // a dependent launch: nothing is read or written before the stream's last kernel
     // has completed
@@ -832,6 +835,10 @@ static __global__ void __launch_bounds__(256)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     for (long long t = blockIdx.x; t < tx * ty; t += gridDim.x) {
         const long long r0 = (t / tx) * TR, c0 = (t % tx) * TC;
+        if (KEEP && threadIdx.x < TR) {
+            const long long r = r0 + threadIdx.x;
+            keep[threadIdx.x] = r < R && __ldg(rowPtr + r) == __ldg(rowPtr + r + 1);
+        }
         if constexpr (VL) {
             float v[4][4];
 #pragma unroll
@@ -872,6 +879,18 @@ static __global__ void __launch_bounds__(256)
                 float o[S];
 #pragma unroll
                 for (int e = 0; e < S; ++e) o[e] = tile[rl + e][cl];
+                if constexpr (KEEP) {
+                    bool any = false;
+#pragma unroll
+                    for (int e = 0; e < S; ++e) any |= keep[rl + e];
+                    if (any) {
+#pragma unroll
+                        for (int e = 0; e < S; ++e)
+                            if (!keep[rl + e])
+                                d[e] = beta == 0.0f ? o[e] : fmaf(beta, d[e], o[e]);
+                        continue;
+                    }
+                }
                 if (beta != 0.0f) {
                     float old[S];
                     ld_plain<S>(old, d);
