@@ -582,6 +582,8 @@ static void run_stream(const Resolved &r, bool cmb, bool cmc, int nr, int nc, in
     a.chunk = r.chunk; a.nchunks = r.nchunks;
     a.meta = (const int2 *)ws;
     a.slots = (float *)((char *)ws + align256(sizeof(int2) * ((size_t)r.nchunks + 1)));
+    static std::atomic<unsigned int> calls{0};
+    a.head_base = ++calls;
     if (nv == 1) {  // one column has no layout
         cmb = cmc = false;
         a.ldb = a.ldc = 1;
@@ -590,7 +592,7 @@ static void run_stream(const Resolved &r, bool cmb, bool cmc, int nr, int nc, in
     if (cmc) launch_stream<true>(r.stream, cmb, a, st);
     else launch_stream<false>(r.stream, cmb, a, st);
     timer_after(st);
-    count_launches(r.nchunks > 1 ? 2 : 1);
+    count_launches(stream_fix_ctas(r.nchunks, nr) > 0 ? 2 : 1);
 }
 
 daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nnz, int nv,

@@ -7,7 +7,10 @@
 // all threads at once (coalesced, several independent loads per thread, no
 // carried state), and only then do threads take rows: one per (row, column) sums
 // its row's products from shared memory in nonzero order, long rows a warp.
-// Rows without nonzeros fall out of the row loop.  A chunk's boundary moves down
+// Rows without nonzeros fall out of the row loop; a chunk with more than kStreamRows rows
+// is left to k_stream_fix, whose warps share out the rows (a million rows, the lower half
+// empty, N = 1 / 8 670 / 2043 us when one CTA walked them, 36 / 88 so; column-major N = 8
+// 6027 and 134).  A chunk's boundary moves down
 // to the start of a row shorter than kStreamSnap; longer rows are cut there, each
 // piece leaves its sum in a slot and k_stream_fix adds the slots in chunk order.
 // No partition pass: two warps of the CTA find the chunk's rows by a 32-way search
@@ -32,6 +35,8 @@ namespace daspmm {
 constexpr int kStreamMaxNv = 8;
 constexpr int kStreamSnap = 64;
 constexpr int kStreamLong = 96;  // nonzeros from which on a warp sums a row
+constexpr int kStreamRows = 4096;  // a chunk of more rows is left to k_stream_fix
+constexpr int kStreamShare = 256;  // rows of a k_stream_fix warp and turn
 
 // Shared memory of a chunk: values, and the rows of B (see pitch in k_stream).
 inline size_t stream_smem(int chunk, int nv, bool cmc)
@@ -142,6 +147,10 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     const int k0 = bound[0].x, r0 = bound[0].y, k1 = bound[1].x, s1 = bound[1].y;
     const bool head = cut[0], tail = cut[1];
     const int rows = s1 - r0 + (tail ? 1 : 0);
+    if (s1 - r0 > kStreamRows) {  // more than one CTA should walk: k_stream_fix's
+        if (t == 0) const_cast<int2 *>(a.meta)[a.nchunks].x = (int)a.head_base;
+        return;
+    }
     auto dest = [&](int row, int k) -> float * {
         if (row == r0 && head) return a.slots + ((size_t)c * 2) * nv + k;
         if (row == s1) return a.slots + ((size_t)c * 2 + 1) * nv + k;
@@ -155,7 +164,8 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     const int fast = CMC ? max(rows, 1) : nv / VC;
     int lo = t % fast, hi = t / fast;
     const int dlo = 256 % fast, dhi = 256 / fast;
-    for (; hi < (CMC ? nv : rows); lo += dlo, hi += dhi + (lo >= fast), lo -= lo >= fast ? fast : 0) {
+    for (; hi < (CMC ? nv : rows);
+         lo += dlo, hi += dhi + (lo >= fast), lo -= lo >= fast ? fast : 0) {
         const int row = r0 + (CMC ? lo : hi), k = CMC ? hi : lo * VC;
         if (CMC && lo >= rows) continue;
         const int p0 = max(__ldg(a.rowPtr + row), k0), p1 = min(__ldg(a.rowPtr + row + 1), k1);
@@ -209,33 +219,138 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     }
 }
 
+// The last chunk whose rows begin at or before `row`, by the whole warp.
+__device__ __forceinline__ int chunk_of(const int2 *meta, int nchunks, int row)
+{
+    const int lane = threadIdx.x & 31;
+    int lo = 0, hi = nchunks;
+    while (hi - lo > 1) {
+        const int step = (hi - lo + 31) / 32, x = lo + (lane + 1) * step;
+        const bool le = x < hi && meta[x].y <= row;
+        const int n = __popc(__ballot_sync(kFull, le));
+        lo += n * step;
+        hi = min(hi, lo + step);
+    }
+    return lo;
+}
+
+// Rows that chunk c begins, up to the next chunk's first: more than kStreamRows?
+__device__ __forceinline__ bool many_rows(const KArgs &a, int c)
+{
+    return (c + 1 < a.nchunks ? a.meta[c + 1].y : a.nr) - a.meta[c].y > kStreamRows;
+}
+
+// What k_stream leaves.
+//
 // Rows cut at chunk boundaries: the warp of the boundary after a row's first piece
 // adds that piece's tail slot and the head slots of the chunks the row reaches.
+//
+// The chunks of more than kStreamRows rows, most of them without nonzeros, which one CTA
+// would walk alone (it says that there are some with the call's number behind the
+// boundaries; an old number there that happens to be this one's costs a look at the
+// boundaries): kStreamShare rows per warp and turn, a lane per row, rows of more than 16
+// nonzeros by the warp.  Only the chunks at a share's two ends can have that many rows.
+// Their pieces of cut rows are summed with the slots of the others.
+//
+// cmb: B is column-major.
 template <bool CMC>
-static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a)
+static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool cmb)
 {
     pdl_trigger();
     pdl_wait();
     const int lane = threadIdx.x & 31, nv = a.nv;
+    const bool left = a.meta[a.nchunks].x == (int)a.head_base;
     const long long c = 1 + (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-    if (c >= a.nchunks) return;
-    const int2 m = a.meta[c], before = a.meta[c - 1];
-    const int rs = __ldg(a.rowPtr + m.y), re = __ldg(a.rowPtr + m.y + 1);
-    if (m.x <= rs || before.x > rs) return;  // no row is cut here, or not for the first time
-    const int last = (re - 1) / a.chunk;     // the chunk of its last piece
+    int2 m = make_int2(0, 0), before = m;
+    int rs = 0, re = 0;
+    if (c < a.nchunks) {
+        m = a.meta[c];
+        before = a.meta[c - 1];
+        rs = __ldg(a.rowPtr + m.y);
+        re = __ldg(a.rowPtr + m.y + 1);
+    }
+    const bool here = m.x > rs && before.x <= rs;  // a row is cut here for the first time
+    if (!here && !left) return;
+    const size_t col_step = cmb ? 1 : a.ldb, k_step = cmb ? a.ldb : 1;
     int kp = 1;
     while (kp < nv) kp <<= 1;
-    const int k = lane & (kp - 1);
-    float x = 0.0f;
-    if (k < nv)
-        for (long long q = c + lane / kp; q <= last; q += 32 / kp)
-            x += __ldcg(a.slots + (q * 2) * nv + k);
-    for (int d = kp; d < 32; d <<= 1) x += __shfl_xor_sync(kFull, x, d);
-    if (lane < kp && k < nv) {
-        x += __ldcg(a.slots + ((c - 1) * 2 + 1) * nv + k);
-        float *p = CMC ? a.C + (size_t)k * a.ldc + m.y : a.C + (size_t)m.y * a.ldc + k;
-        *p = a.beta == 0.0f ? x : fmaf(a.beta, *p, x);
+    const int k = lane & (kp - 1), sub = lane / kp, subs = 32 / kp;
+    auto term = [&](float x, int p, int col) {
+        return fmaf(__ldg(a.vals + p),
+                    __ldg(a.B + __ldg(a.colIdx + p) * col_step + col * k_step), x);
+    };
+    // nonzeros [p0, p1) of a row, this lane's share of them in its column
+    auto piece = [&](float x, int p0, int p1) {
+        for (int p = p0 + sub; p < p1; p += subs) x = term(x, p, k);
+        return x;
+    };
+    auto store = [&](int row, int col, float x, bool holds) {
+        float *d = CMC ? a.C + (size_t)col * a.ldc + row : a.C + (size_t)row * a.ldc + col;
+        if (a.beta == 0.0f) *d = x;
+        else if (a.beta != 1.0f || holds) *d = fmaf(a.beta, *d, x);
+    };
+    if (here) {
+        int last = min((re - 1) / a.chunk, a.nchunks - 1);  // the chunk of its last piece
+        const bool first_left = m.y - before.y > kStreamRows, last_left = many_rows(a, last);
+        float x = 0.0f;
+        if (k < nv) {
+            if (last_left) x = piece(x, last * a.chunk, re);
+            if (first_left) x = piece(x, rs, m.x);
+            for (long long q = c + sub; q <= last - last_left; q += subs)
+                x += __ldcg(a.slots + (q * 2) * nv + k);
+        }
+        for (int d = kp; d < 32; d <<= 1) x += __shfl_xor_sync(kFull, x, d);
+        if (lane < kp && k < nv) {
+            if (!first_left) x += __ldcg(a.slots + ((c - 1) * 2 + 1) * nv + k);
+            store(m.y, k, x, true);
+        }
     }
+    if (!left) return;
+    const int nwarps = (int)gridDim.x * 8, w = (int)blockIdx.x * 8 + (threadIdx.x >> 5);
+    for (long long b = (long long)w * kStreamShare; b < a.nr; b += (long long)nwarps * kStreamShare) {
+        const int a0 = (int)b, a1 = (int)min((long long)a.nr, b + kStreamShare);
+        for (int at = a0; at < a1;) {
+            const int h = chunk_of(a.meta, a.nchunks, at);
+            const int2 m = a.meta[h];
+            const int next = h + 1 < a.nchunks ? a.meta[h + 1].y : a.nr;
+            // (its first row may be the last piece of a cut one)
+            const int begin = max(a0, m.y + (m.x > __ldg(a.rowPtr + m.y) ? 1 : 0));
+            const int end = next - m.y > kStreamRows ? min(a1, next) : 0;
+            for (int r0 = begin; r0 < end; r0 += 32) {
+                const int row = r0 + lane;
+                int p0 = 0, p1 = 0;
+                if (row < end) {
+                    p0 = __ldg(a.rowPtr + row);
+                    p1 = __ldg(a.rowPtr + row + 1);
+                }
+                if (row < end && p1 - p0 <= 16) {
+                    for (int col = 0; col < nv; ++col) {
+                        float x = 0.0f;
+                        for (int p = p0; p < p1; ++p) x = term(x, p, col);
+                        store(row, col, x, p0 < p1);
+                    }
+                }
+                for (unsigned more = __ballot_sync(kFull, p1 - p0 > 16); more; more &= more - 1) {
+                    const int l = __ffs(more) - 1;
+                    const int q0 = __shfl_sync(kFull, p0, l), q1 = __shfl_sync(kFull, p1, l);
+                    float x = k < nv ? piece(0.0f, q0, q1) : 0.0f;
+                    for (int d = kp; d < 32; d <<= 1) x += __shfl_xor_sync(kFull, x, d);
+                    if (lane < kp && k < nv) store(r0 + l, k, x, true);
+                }
+            }
+            at = next >= a1 ? a1 : max(at + 1, a1 - 1);
+        }
+    }
+}
+
+// The CTAs of k_stream_fix: eight boundaries each, and enough for the rows that may be
+// left (no chunk of fewer rows has more than kStreamRows).
+inline int stream_fix_ctas(int nchunks, int nr)
+{
+    const int cuts = (nchunks - 1 + 7) / 8;
+    if (nr <= kStreamRows) return cuts;
+    return std::max(cuts, std::min((nr + 8 * kStreamShare - 1) / (8 * kStreamShare),
+                                   device_sms() * 4));
 }
 
 // Nonzeros per chunk: one wave of eight CTAs per SM, in steps of 128, at most what
@@ -268,10 +383,11 @@ inline void launch_stream_as(const KArgs &a, cudaStream_t st)
     cfg.numAttrs = 1;
     cudaLaunchKernelEx(&cfg, a.beta == 1.0f ? k_stream<NV, V, CMB, CMC, true>
                                             : k_stream<NV, V, CMB, CMC, false>, a);
-    if (a.nchunks > 1) {
-        cfg.gridDim = dim3((unsigned)((a.nchunks - 1 + 7) / 8));
+    const int fix = stream_fix_ctas(a.nchunks, a.nr);
+    if (fix > 0) {
+        cfg.gridDim = dim3((unsigned)fix);
         cfg.dynamicSmemBytes = 0;
-        cudaLaunchKernelEx(&cfg, k_stream_fix<CMC>, a);
+        cudaLaunchKernelEx(&cfg, k_stream_fix<CMC>, a, CMB);
     }
 }
 
