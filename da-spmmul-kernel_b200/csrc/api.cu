@@ -558,6 +558,22 @@ static void launch_transpose(const float *src, long long R, long long Cn, float 
     count_launches(1);
 }
 
+static void launch_coo_rows(int nr, int nnz, const int *rowIdx, int *rowPtr, int chunk, int2 *meta,
+                            cudaStream_t st)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(((long long)nnz + 1 + 255) / 256));
+    cfg.blockDim = dim3(256);
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_coo_rows, nr, nnz, rowIdx, rowPtr, chunk, meta);
+    count_launches(1);
+}
+
 static unsigned grid_x(long long units, int G, int block)
 {
     const long long gpb = (long long)(block / 32) * (32 / G);
@@ -1005,18 +1021,8 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
             bounds += align256(sizeof(float) * (size_t)nc * nv) +
                       align256(sizeof(float) * (size_t)nr * nv);
         }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)(((long long)nnz + 1 + 255) / 256));
-        cfg.blockDim = dim3(256);
-        cfg.stream = st;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        at[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_coo_rows, nr, nnz, rowIdx, (int *)ws, (int)in.chunk,
-                           in.stream ? (int2 *)nullptr : (int2 *)bounds);
-        count_launches(1);
+        launch_coo_rows(nr, nnz, rowIdx, (int *)ws, in.chunk, in.stream ? nullptr : (int2 *)bounds,
+                        st);
         rowPtr = (const int *)ws;
     }
     *done = true;
@@ -1183,10 +1189,7 @@ daspmm_status daspmm_ownership(int alg, int nr, int nnz, const int *rowPtr, cons
 daspmm_status daspmm_coo_to_csr(int nr, int nnz, const int *rowIdx, int *rowPtr, void *stream)
 {
     if (nr < 0 || nnz < 0 || !rowPtr || (nnz > 0 && !rowIdx)) return DASPMM_ERR_INVALID;
-    const long long n = (long long)nnz + 1;
-    const unsigned g = (unsigned)std::max<long long>(1, (n + 255) / 256);
-    k_coo_to_csr<<<g, 256, 0, (cudaStream_t)stream>>>(nr, nnz, rowIdx, rowPtr);
-    count_launches(1);
+    launch_coo_rows(nr, nnz, rowIdx, rowPtr, 1, nullptr, (cudaStream_t)stream);
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? DASPMM_OK : cuda_fail(e);
 }

@@ -913,33 +913,35 @@ static __global__ void k_scale(float *C, size_t n, float beta)
         C[i] = beta == 0.0f ? 0.0f : beta * C[i];
 }
 
-// rowPtr[r] = number of nonzeros with row < r, from sorted COO rows: every
-// nonzero p whose row differs from its predecessor's fills the pointers of
-// the rows in between (empty rows included).  Bit-exact with
-// generateCsrRowPtrArray (spmvspmm_benchmark.cu:41-76).
-static __global__ void k_coo_to_csr(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr)
-{
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > nnz) return;
-    const int prev = p == 0 ? -1 : __ldg(rowIdx + p - 1);
-    const int cur = p == nnz ? nr : __ldg(rowIdx + p);
-    for (int r = prev + 1; r <= cur && r <= nr; ++r) rowPtr[r] = (int)p;
-}
-
-// The same, and boundaries that are in range whatever the rows are (k_partition
-// writes the balanced split's over them; of rows that do not ascend it would leave
-// some unwritten).  Launched as a dependent of the stream's previous kernel.
-static __global__ void k_coo_rows(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr,
-                                  int chunk, int2 *meta)
+// Row pointer of sorted rows (COO): rowPtr[r] = the first nonzero at or behind row r.  A
+// thread per nonzero p, and one past the last, fills what lies between its row and the one
+// before; of a longer run of empty rows the first kCooRun entries, and its warp together the
+// rest (a million rows with one run of all of them 3673 us by one thread, 125 so; with a
+// thousand nonzeros 148 and 31).  Bit-exact with generateCsrRowPtrArray
+// (spmvspmm_benchmark.cu:41-76).  Launched as a dependent of the stream's previous kernel.
+// With `meta`, also boundaries that are in range whatever the rows are (k_partition writes
+// the balanced split's over them; of rows that do not ascend it would leave some unwritten).
+constexpr int kCooRun = 32;
+static __global__ void __launch_bounds__(256)
+    k_coo_rows(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr, int chunk, int2 *meta)
 {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p > nnz) return;
-    const int prev = p == 0 ? -1 : __ldg(rowIdx + p - 1);
-    const int cur = p == nnz ? nr : __ldg(rowIdx + p);
-    for (int r = prev + 1; r <= cur && r <= nr; ++r) rowPtr[r] = (int)p;
-    if (meta && p < nnz && p % chunk == 0) meta[p / chunk] = make_int2((int)p, cur);
+    const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+    int own = 0, to = 0;
+    if (p <= nnz) {
+        const int prev = p == 0 ? -1 : __ldg(rowIdx + p - 1);
+        const int cur = p == nnz ? nr : __ldg(rowIdx + p);
+        to = min(cur, nr);
+        own = (int)min((long long)to, (long long)prev + kCooRun);
+        for (int r = prev + 1; r <= own; ++r) rowPtr[r] = (int)p;
+        if (meta && p < nnz && p % chunk == 0) meta[p / chunk] = make_int2((int)p, cur);
+    }
+    for (unsigned more = __ballot_sync(kFull, own < to); more; more &= more - 1) {
+        const int l = __ffs(more) - 1, r0 = __shfl_sync(kFull, own, l) + 1;
+        const int r1 = __shfl_sync(kFull, to, l), v = (int)__shfl_sync(kFull, (int)p, l);
+        for (int r = r0 + (int)(threadIdx.x & 31); r <= r1; r += 32) rowPtr[r] = v;
+    }
 }
 
 // Ownership recording buffers (tests): owner = INT_MAX / pieces = 0, then
