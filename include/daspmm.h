@@ -120,7 +120,7 @@ daspmm_status daspmm_spmm_ex(const daspmm_config *cfg, int layout, int nr, int n
                              void *stream);
 
 /* Gives the idle memory of the current device's scratch pool back to the device, down
- * to `keep` bytes (at most 512 MiB stay there otherwise).  No counterpart in the
+ * to `keep` bytes (up to 2 GiB stay there otherwise).  No counterpart in the
  * reference, which allocates nothing. */
 daspmm_status daspmm_scratch_trim(size_t keep);
 
