@@ -562,7 +562,8 @@ static void launch_coo_rows(int nr, int nnz, const int *rowIdx, int *rowPtr, int
                             cudaStream_t st)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(((long long)nnz + 1 + 255) / 256));
+    const int far = nr / kCooFar;
+    cfg.gridDim = dim3((unsigned)far + (unsigned)(((long long)nnz + 1 + 255) / 256));
     cfg.blockDim = dim3(256);
     cfg.stream = st;
     cudaLaunchAttribute at[1];
@@ -570,7 +571,7 @@ static void launch_coo_rows(int nr, int nnz, const int *rowIdx, int *rowPtr, int
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_coo_rows, nr, nnz, rowIdx, rowPtr, chunk, meta);
+    cudaLaunchKernelEx(&cfg, k_coo_rows, nr, nnz, rowIdx, rowPtr, chunk, meta, far);
     count_launches(1);
 }
 

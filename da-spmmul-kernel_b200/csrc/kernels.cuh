@@ -915,32 +915,54 @@ static __global__ void k_scale(float *C, size_t n, float beta)
 
 // Row pointer of sorted rows (COO): rowPtr[r] = the first nonzero at or behind row r.  A
 // thread per nonzero p, and one past the last, fills what lies between its row and the one
-// before; of a longer run of empty rows the first kCooRun entries, and its warp together the
-// rest (a million rows with one run of all of them 3673 us by one thread, 125 so; with a
-// thousand nonzeros 148 and 31).  Bit-exact with generateCsrRowPtrArray
+// before; of a longer run of empty rows the first kCooRun entries, its warp together the
+// next ones up to kCooFar, and the first `far` CTAs what is further, kCooFar entries each
+// from kCooFar on, by a 32-way search (they come first because of its latency).  A million
+// rows with one run of all of them 3673 us by one thread, 5.6 so; with a thousand nonzeros
+// 148 and 28; 262k power-law rows 6.2 and 6.4.  Bit-exact with generateCsrRowPtrArray
 // (spmvspmm_benchmark.cu:41-76).  Launched as a dependent of the stream's previous kernel.
 // With `meta`, also boundaries that are in range whatever the rows are (k_partition writes
 // the balanced split's over them; of rows that do not ascend it would leave some unwritten).
-constexpr int kCooRun = 32;
+constexpr int kCooRun = 32, kCooFar = 4096;
 static __global__ void __launch_bounds__(256)
-    k_coo_rows(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr, int chunk, int2 *meta)
+    k_coo_rows(int nr, int nnz, const int *__restrict__ rowIdx, int *rowPtr, int chunk, int2 *meta,
+               int far)
 {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const long long p = (long long)blockIdx.x * 256 + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    if ((int)blockIdx.x < far) {
+        const int first = ((int)blockIdx.x + 1) * kCooFar;  // <= nr
+        int lo = 0, hi = nnz;  // the first nonzero at or behind row `first` lies in [lo, hi]
+        while (lo < hi) {
+            const int step = (hi - lo + 31) / 32;
+            const long long x = (long long)lo + (long long)(lane + 1) * step - 1;
+            const bool before = x < hi && __ldg(rowIdx + x) < first;
+            lo += __popc(__ballot_sync(kFull, before)) * step;
+            hi = min(hi, lo + step - 1);
+        }
+        const int prev = lo == 0 ? -1 : __ldg(rowIdx + lo - 1);
+        const int cur = lo == nnz ? nr : __ldg(rowIdx + lo);
+        const int to = min(min(cur, nr), first + min(kCooFar - 1, nr - first));
+        for (long long r = max((long long)first, (long long)prev + 1 + kCooFar) + threadIdx.x;
+             r <= to; r += 256)
+            rowPtr[r] = lo;
+        return;
+    }
+    const long long p = (long long)((int)blockIdx.x - far) * 256 + threadIdx.x;
     int own = 0, to = 0;
     if (p <= nnz) {
         const int prev = p == 0 ? -1 : __ldg(rowIdx + p - 1);
         const int cur = p == nnz ? nr : __ldg(rowIdx + p);
-        to = min(cur, nr);
+        to = (int)min((long long)min(cur, nr), (long long)prev + kCooFar);
         own = (int)min((long long)to, (long long)prev + kCooRun);
         for (int r = prev + 1; r <= own; ++r) rowPtr[r] = (int)p;
         if (meta && p < nnz && p % chunk == 0) meta[p / chunk] = make_int2((int)p, cur);
     }
     for (unsigned more = __ballot_sync(kFull, own < to); more; more &= more - 1) {
         const int l = __ffs(more) - 1, r0 = __shfl_sync(kFull, own, l) + 1;
-        const int r1 = __shfl_sync(kFull, to, l), v = (int)__shfl_sync(kFull, (int)p, l);
-        for (int r = r0 + (int)(threadIdx.x & 31); r <= r1; r += 32) rowPtr[r] = v;
+        const int r1 = __shfl_sync(kFull, to, l), v = __shfl_sync(kFull, (int)p, l);
+        for (int r = r0 + lane; r <= r1; r += 32) rowPtr[r] = v;
     }
 }
 

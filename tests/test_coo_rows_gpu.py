@@ -7,7 +7,7 @@ import daspmm as D
 from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
-RUN = 32   # entries that one thread fills
+RUN, FAR = 32, 4096   # entries that one thread fills, and its warp
 
 
 def _rows(case):
@@ -15,7 +15,7 @@ def _rows(case):
     if case == "none":
         return 1000, np.zeros(0, np.int32)
     if case == "edges":   # runs of RUN - 2 .. RUN + 2 empty rows, and of many
-        lens = [x + d for x in (RUN, 256, RUN + 256, 1000) for d in (-2, -1, 0, 1, 2)] + [9000, 9001]
+        lens = [x + d for x in (RUN, 256, FAR, 2 * FAR) for d in (-2, -1, 0, 1, 2)] + [9000, 9001]
         at = np.cumsum([x + 1 for x in lens * 3])
         return int(at[-1]) + 1 + RUN, np.repeat(at, rng.integers(1, 40, at.size)).astype(np.int32)
     if case == "front":
