@@ -8,10 +8,9 @@
 // carried state), and only then do threads take rows: one per (row, column) sums
 // its row's products from shared memory in nonzero order, long rows a warp.
 // Rows without nonzeros fall out of the row loop; a chunk with more than kStreamRows rows
-// is left to k_stream_fix, whose warps share out the rows (a million rows, the lower half
-// empty, N = 1 / 8 670 / 2043 us when one CTA walked them, 36 / 88 so; column-major N = 8
-// 6027 and 134).  A chunk's boundary moves down
-// to the start of a row shorter than kStreamSnap; longer rows are cut there, each
+// is left to k_stream_fix, whose warps share out the rows (a million rows of 8, the lower
+// half empty, N = 1 / 8 670 / 2043 us when one CTA walked them, 37 / 65 so; column-major
+// N = 8 6027 and 128).  A chunk's boundary moves down to the start of a row shorter than kStreamSnap; longer rows are cut there, each
 // piece leaves its sum in a slot and k_stream_fix adds the slots in chunk order.
 // No partition pass: two warps of the CTA find the chunk's rows by a 32-way search
 // while the others load (so the chunk's load starts kStreamSnap - 1 nonzeros
@@ -36,7 +35,6 @@ constexpr int kStreamMaxNv = 8;
 constexpr int kStreamSnap = 64;
 constexpr int kStreamLong = 96;  // nonzeros from which on a warp sums a row
 constexpr int kStreamRows = 4096;  // a chunk of more rows is left to k_stream_fix
-constexpr int kStreamShare = 256;  // rows of a k_stream_fix warp and turn
 
 // Shared memory of a chunk: values, and the rows of B (see pitch in k_stream).
 inline size_t stream_smem(int chunk, int nv, bool cmc)
@@ -219,21 +217,6 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     }
 }
 
-// The last chunk whose rows begin at or before `row`, by the whole warp.
-__device__ __forceinline__ int chunk_of(const int2 *meta, int nchunks, int row)
-{
-    const int lane = threadIdx.x & 31;
-    int lo = 0, hi = nchunks;
-    while (hi - lo > 1) {
-        const int step = (hi - lo + 31) / 32, x = lo + (lane + 1) * step;
-        const bool le = x < hi && meta[x].y <= row;
-        const int n = __popc(__ballot_sync(kFull, le));
-        lo += n * step;
-        hi = min(hi, lo + step);
-    }
-    return lo;
-}
-
 // Rows that chunk c begins, up to the next chunk's first: more than kStreamRows?
 __device__ __forceinline__ bool many_rows(const KArgs &a, int c)
 {
@@ -248,9 +231,8 @@ __device__ __forceinline__ bool many_rows(const KArgs &a, int c)
 // The chunks of more than kStreamRows rows, most of them without nonzeros, which one CTA
 // would walk alone (it says that there are some with the call's number behind the
 // boundaries; an old number there that happens to be this one's costs a look at the
-// boundaries): kStreamShare rows per warp and turn, a lane per row, rows of more than 16
-// nonzeros by the warp.  Only the chunks at a share's two ends can have that many rows.
-// Their pieces of cut rows are summed with the slots of the others.
+// boundaries): 32 rows per warp and turn, a lane per row, rows of more than 16 nonzeros by
+// the warp.  Their pieces of cut rows are summed with the slots of the others.
 //
 // cmb: B is column-major.
 template <bool CMC>
@@ -275,13 +257,11 @@ static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool c
     int kp = 1;
     while (kp < nv) kp <<= 1;
     const int k = lane & (kp - 1), sub = lane / kp, subs = 32 / kp;
-    auto term = [&](float x, int p, int col) {
-        return fmaf(__ldg(a.vals + p),
-                    __ldg(a.B + __ldg(a.colIdx + p) * col_step + col * k_step), x);
-    };
     // nonzeros [p0, p1) of a row, this lane's share of them in its column
     auto piece = [&](float x, int p0, int p1) {
-        for (int p = p0 + sub; p < p1; p += subs) x = term(x, p, k);
+        for (int p = p0 + sub; p < p1; p += subs)
+            x = fmaf(__ldg(a.vals + p),
+                     __ldg(a.B + __ldg(a.colIdx + p) * col_step + k * k_step), x);
         return x;
     };
     auto store = [&](int row, int col, float x, bool holds) {
@@ -307,38 +287,62 @@ static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool c
     }
     if (!left) return;
     const int nwarps = (int)gridDim.x * 8, w = (int)blockIdx.x * 8 + (threadIdx.x >> 5);
-    for (long long b = (long long)w * kStreamShare; b < a.nr; b += (long long)nwarps * kStreamShare) {
-        const int a0 = (int)b, a1 = (int)min((long long)a.nr, b + kStreamShare);
-        for (int at = a0; at < a1;) {
-            const int h = chunk_of(a.meta, a.nchunks, at);
-            const int2 m = a.meta[h];
-            const int next = h + 1 < a.nchunks ? a.meta[h + 1].y : a.nr;
-            // (its first row may be the last piece of a cut one)
-            const int begin = max(a0, m.y + (m.x > __ldg(a.rowPtr + m.y) ? 1 : 0));
-            const int end = next - m.y > kStreamRows ? min(a1, next) : 0;
-            for (int r0 = begin; r0 < end; r0 += 32) {
-                const int row = r0 + lane;
-                int p0 = 0, p1 = 0;
-                if (row < end) {
-                    p0 = __ldg(a.rowPtr + row);
-                    p1 = __ldg(a.rowPtr + row + 1);
-                }
-                if (row < end && p1 - p0 <= 16) {
-                    for (int col = 0; col < nv; ++col) {
-                        float x = 0.0f;
-                        for (int p = p0; p < p1; ++p) x = term(x, p, col);
-                        store(row, col, x, p0 < p1);
-                    }
-                }
-                for (unsigned more = __ballot_sync(kFull, p1 - p0 > 16); more; more &= more - 1) {
-                    const int l = __ffs(more) - 1;
-                    const int q0 = __shfl_sync(kFull, p0, l), q1 = __shfl_sync(kFull, p1, l);
-                    float x = k < nv ? piece(0.0f, q0, q1) : 0.0f;
-                    for (int d = kp; d < 32; d <<= 1) x += __shfl_xor_sync(kFull, x, d);
-                    if (lane < kp && k < nv) store(r0 + l, k, x, true);
-                }
+    constexpr int T = 4;  // groups of 32 rows in flight, nwarps apart: those that hold
+                          // something lie next to each other, and so on different warps
+    for (long long b = 32LL * w; b < a.nr; b += 32LL * T * nwarps) {
+        int p0[T], len[T];
+        int2 m[T];
+        int next[T];
+#pragma unroll
+        for (int g = 0; g < T; ++g) {
+            const long long row = b + 32LL * g * nwarps + lane;
+            p0[g] = row < a.nr ? __ldg(a.rowPtr + row) : 0;
+            len[g] = row < a.nr ? __ldg(a.rowPtr + row + 1) - p0[g] : -1;
+        }
+        // Chunk c begins in the row of nonzero c * chunk, so a row lies in the chunk of the
+        // last nonzero of the rows up to it.
+#pragma unroll
+        for (int g = 0; g < T; ++g) {
+            const int h = min(max(p0[g] + max(len[g], 0) - 1, 0) / a.chunk, a.nchunks - 1);
+            m[g] = a.meta[h];
+            next[g] = h + 1 < a.nchunks ? a.meta[h + 1].y : a.nr;
+        }
+#pragma unroll
+        for (int g = 0; g < T; ++g) {
+            const long long r0 = b + 32LL * g * nwarps;
+            const int row = (int)(r0 + lane);
+            // of a chunk with too many rows; the chunk's first may be the last piece of a cut one
+            if (next[g] - m[g].y <= kStreamRows || (row == m[g].y && m[g].x > p0[g])) len[g] = -1;
+            const bool none = __all_sync(kFull, len[g] == 0);
+            if (none && a.beta == 1.0f) continue;
+            if (!CMC && none) {  // nothing in 32 rows: whole lines of beta*C
+                float *d = a.C + (size_t)r0 * a.ldc;
+                for (int i = lane; i < 32 * nv; i += 32)
+                    d[i] = a.beta == 0.0f ? 0.0f : fmaf(a.beta, d[i], 0.0f);
+                continue;
             }
-            at = next >= a1 ? a1 : max(at + 1, a1 - 1);
+            if (len[g] >= 0 && len[g] <= 16) {
+                float x[kStreamMaxNv];
+#pragma unroll
+                for (int e = 0; e < kStreamMaxNv; ++e) x[e] = 0.0f;
+                for (int p = p0[g]; p < p0[g] + len[g]; ++p) {
+                    const float v = __ldg(a.vals + p);
+                    const float *bp = a.B + __ldg(a.colIdx + p) * col_step;
+#pragma unroll
+                    for (int e = 0; e < kStreamMaxNv; ++e)
+                        if (e < nv) x[e] = fmaf(v, __ldg(bp + e * k_step), x[e]);
+                }
+#pragma unroll
+                for (int e = 0; e < kStreamMaxNv; ++e)
+                    if (e < nv) store(row, e, x[e], len[g] > 0);
+            }
+            for (unsigned more = __ballot_sync(kFull, len[g] > 16); more; more &= more - 1) {
+                const int l = __ffs(more) - 1;
+                const int q0 = __shfl_sync(kFull, p0[g], l), q1 = q0 + __shfl_sync(kFull, len[g], l);
+                float x = k < nv ? piece(0.0f, q0, q1) : 0.0f;
+                for (int d = kp; d < 32; d <<= 1) x += __shfl_xor_sync(kFull, x, d);
+                if (lane < kp && k < nv) store((int)r0 + l, k, x, true);
+            }
         }
     }
 }
@@ -349,8 +353,7 @@ inline int stream_fix_ctas(int nchunks, int nr)
 {
     const int cuts = (nchunks - 1 + 7) / 8;
     if (nr <= kStreamRows) return cuts;
-    return std::max(cuts, std::min((nr + 8 * kStreamShare - 1) / (8 * kStreamShare),
-                                   device_sms() * 4));
+    return std::max(cuts, std::min(nr / 2048 + 1, device_sms() * 4));
 }
 
 // Nonzeros per chunk: one wave of eight CTAs per SM, in steps of 128, at most what
