@@ -982,22 +982,34 @@ public:
 //               random 262k x 2, N = 16 29 -> 44, N = 64 119 -> 62; vector, random 65k x 2,
 //               N = 64 31 -> 35; vector at N <= 8 reads A as fast: 262k x 24, N = 1 62 -> 67,
 //               262k x 8 29 -> 26; vector, random 4k x 24, N = 16 17 -> 19, 16k x 24 27 -> 22
+// With far more rows than nonzeros the own kernels cost what their rows (CSR) or their
+// nonzeros (COO) do, while the window kernel seeks each nonzero's row: random 131k rows of
+// 0.25, N = 16, CSR scalar 8.7 -> 56, CSR vector 35 -> 56, COO 25 / 21 -> 57; of 1 25 / 21
+// -> 35 and 37 -> 30 (CSR vector); of 2 13 -> 17, 39 -> 17, 25 / 23 -> 26.
+// AUTO's other choice is CSR scalar, which wins by a few us on small calls with even rows
+// and loses by factors where rows are not even (4k x 2, N = 1 uniform 7.5 and 10.5, power-law 45
+// and 11; 262k x 8, N = 8 uniform 15 and 29, power-law 335 and 37): only the rows decide.
 static bool balanced_pays(int alg, bool cm, int nr, int nnz, int nv)
 {
     const long long out = (long long)nr * nv;
     const bool sparse = nnz < 4LL * nr;
+    const bool one = nnz >= (long long)nr, more = 2LL * nnz >= 3LL * nr;  // nonzeros per row
     switch (alg) {
     case DASPMM_ALG_CSR_SCALAR:
-        return cm ? nv >= 16 && out >= (1 << 22) : nv >= 32 && out >= (1 << 23);
+        return more && (cm ? nv >= 16 && out >= (1 << 22) : nv >= 32 && out >= (1 << 23));
     case DASPMM_ALG_CSR_VECTOR:
-        return nr >= 65536 || out >= (cm ? 1 << 18 : 1 << 21);
+        return (one || nv <= kStreamMaxNv) &&
+               (nr >= 65536 || out >= (cm ? 1 << 18 : 1 << 21));
     case DASPMM_ALG_AUTO:
-        return true;
+        return nv <= kStreamMaxNv ? one : more;
     case DASPMM_ALG_COO_SCALAR:
-        return cm || nv <= kStreamMaxNv || nv >= 64 || !sparse || out >= (1 << 23);
+        if (nv <= kStreamMaxNv) return 4LL * nnz >= nr;
+        return one && (cm || nv >= 64 || !sparse || (more && out >= (1 << 23)));
     default:
-        if (nv <= kStreamMaxNv) return (cm && nv > 1) || nnz < (1 << 22);
-        return cm || out >= (sparse ? 1 << 23 : 1 << 18) || (!sparse && nv >= 64);
+        if (nv <= kStreamMaxNv)
+            return one && ((cm && nv > 2) || nnz < (nv <= 2 ? 1 << 21 : 1 << 22));
+        if (cm) return one;
+        return more && (out >= (sparse ? 1 << 23 : 1 << 18) || (!sparse && nv >= 64));
     }
 }
 
