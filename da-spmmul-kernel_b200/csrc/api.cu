@@ -597,6 +597,7 @@ static void run_stream(const Resolved &r, bool cmb, bool cmc, int nr, int nc, in
     a.rowPtr = rowPtr; a.colIdx = colIdx; a.vals = values;
     a.B = B; a.C = C; a.beta = beta;
     a.chunk = r.chunk; a.nchunks = r.nchunks;
+    a.based = r.based;
     a.meta = (const int2 *)ws;
     a.slots = (float *)((char *)ws + align256(sizeof(int2) * ((size_t)r.nchunks + 1)));
     static std::atomic<unsigned int> calls{0};
@@ -633,6 +634,7 @@ daspmm_status run_resolved(const Resolved &r, int layout, int nr, int nc, int nn
         Resolved in;
         daspmm_status s = resolve_inner(r, nv, Brm, Crm, &in);
         if (s != DASPMM_OK) return s;
+        in.based = r.based;
         // B column-major = an nv x nc row-major array; its transpose is row-major B
         launch_transpose(B, nv, nc, Brm, 0.0f, st);
         if (in.stream) {
@@ -778,7 +780,7 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_partition, nr, nnz, rowPtr, (int)r.chunk, (int)r.snap,
+    cudaLaunchKernelEx(&cfg, r.based ? k_partition<true> : k_partition<false>, nr, nnz, rowPtr, (int)r.chunk, (int)r.snap,
                        (int)r.nchunks, const_cast<int2 *>(a.meta), a.cnt, (int)r.tiles, a.head,
                        a.emap, rows_beta && a.beta != 1.0f ? a.C : (float *)nullptr, a.nv, a.beta);
     count_launches(1);
@@ -1055,6 +1057,9 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
                         st);
         rowPtr = (const int *)ws;
     }
+    // The CSR kernels ask nothing of rowPtr[0] and nnz: rows r.. of a larger matrix are
+    // rowPtr + r with its colIdx and values.
+    r.based = !coo;
     *done = true;
     return run_resolved(r, layout, nr, nc, nnz, nv, rowPtr, nullptr, colIdx, values, B, C, beta,
                         own, need, st);
@@ -1171,7 +1176,7 @@ daspmm_status daspmm_partition(int nr, int nnz, const int *rowPtr, int chunk, in
     if (nr < 0 || nnz < 0 || chunk < 1 || snap < 1 || !rowPtr || !meta) return DASPMM_ERR_INVALID;
     const int nch = daspmm_num_chunks(nnz, chunk);
     const unsigned pg = (unsigned)std::max(1, (nr + 255) / 256);
-    k_partition<<<pg, 256, 0, (cudaStream_t)stream>>>(nr, nnz, rowPtr, chunk, std::min(snap, chunk),
+    k_partition<><<<pg, 256, 0, (cudaStream_t)stream>>>(nr, nnz, rowPtr, chunk, std::min(snap, chunk),
                                                       nch, (int2 *)meta, nullptr, 1, nullptr,
                                                       nullptr, nullptr, 0, 0.0f);
     count_launches(1);

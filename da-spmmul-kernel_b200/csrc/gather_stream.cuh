@@ -34,6 +34,7 @@ namespace daspmm {
 constexpr int kStreamMaxNv = 8;
 constexpr int kStreamSnap = 64;
 constexpr int kStreamLong = 96;  // nonzeros from which on a warp sums a row
+constexpr int kStreamPlain = 0, kStreamOne = 1, kStreamBased = 2;  // see k_stream
 constexpr int kStreamRows = 4096;  // a chunk of more rows is left to k_stream_fix
 
 // Shared memory of a chunk: values, and the rows of B (see pitch in k_stream).
@@ -59,10 +60,12 @@ __device__ __forceinline__ int row_of(const int *__restrict__ rowPtr, int nr, in
 }
 
 // NV: nv where it is known at compile time, else 0.  V floats per load of B (nv % V
-// == 0, B aligned to them).  CMB / CMC: B / C column-major (B only with V == 1).  ONE: beta
-// is 1, so a row without nonzeros is C's already and not touched (a form of its own: the
-// check in one form for all cost 1 % at one and eight columns).
-template <int NV, int V, bool CMB, bool CMC, bool ONE>
+// == 0, B aligned to them).  CMB / CMC: B / C column-major (B only with V == 1).  KIND, of
+// which each is a form of its own because the checks in one for all cost 1 to 10 % at one
+// and eight columns: kStreamOne, beta is 1, so a row without nonzeros is C's already and not
+// touched; kStreamBased, the rows are some of a larger matrix's, whose row pointer does not
+// start at 0 and whose nnz may be the matrix's.
+template <int NV, int V, bool CMB, bool CMC, int KIND>
 __global__ void __launch_bounds__(256) k_stream(const KArgs a)
 {
     extern __shared__ __align__(16) float stream_mem[];
@@ -78,17 +81,21 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     const uint64_t pol_once = policy_evict_first();
     pdl_trigger();
     pdl_wait();
-    const long long kn0 = (long long)c * a.chunk;
-    const int kn1 = (int)min((long long)a.nnz, kn0 + a.chunk);
-    const int klo = c == 0 ? 0 : (int)kn0 - (kStreamSnap - 1);  // chunk >= kStreamSnap
+    constexpr bool BASED = KIND == kStreamBased;
+    const int base = BASED ? __ldg(a.rowPtr) : 0, stop = BASED ? __ldg(a.rowPtr + a.nr) : a.nnz;
+    long long kn0 = (long long)c * a.chunk;
+    if (BASED) kn0 = min((long long)stop, base + kn0);
+    const int kn1 = (int)min((long long)stop, kn0 + a.chunk);
+    const int klo = BASED ? max(base, (int)kn0 - (kStreamSnap - 1))
+                          : c == 0 ? 0 : (int)kn0 - (kStreamSnap - 1);  // chunk >= kStreamSnap
     const int n = kn1 - klo;
     float *sb = stream_mem, *sv = stream_mem + (a.chunk + kStreamSnap) * pitch;
     if (t == 0) nlong = 0;
     if (warp < 2) {  // these find the chunk's rows, the others load
         const int k = warp == 0 ? (int)kn0 : kn1;
-        int2 m = make_int2(k, warp == 0 ? 0 : a.nr);
+        int2 m = make_int2(k, warp == 0 && (!BASED || c == 0) ? 0 : a.nr);
         bool across = false;
-        if (warp == 0 ? c > 0 : k < a.nnz) {
+        if (BASED ? k < stop && (warp == 1 || c > 0) : warp == 0 ? c > 0 : k < a.nnz) {
             const int r = row_of(a.rowPtr, a.nr, k);
             const int rs = __ldg(a.rowPtr + r), re = __ldg(a.rowPtr + r + 1);
             // (never before the chunk's load begins, whatever the row pointer says)
@@ -158,7 +165,7 @@ __global__ void __launch_bounds__(256) k_stream(const KArgs a)
     // (row, VC columns) of thread t, then every 256 further: row-major, columns next to
     // each other, so a warp stores whole lines; column-major, rows.
     constexpr int VC = CMC ? 1 : V;
-    constexpr int least = ONE ? 1 : 0;  // nonzeros of the rows that are written
+    constexpr int least = KIND == kStreamOne ? 1 : 0;  // nonzeros of the rows that are written
     const int fast = CMC ? max(rows, 1) : nv / VC;
     int lo = t % fast, hi = t / fast;
     const int dlo = 256 % fast, dhi = 256 / fast;
@@ -248,11 +255,16 @@ static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool c
     if (c < a.nchunks) {
         m = a.meta[c];
         before = a.meta[c - 1];
-        rs = __ldg(a.rowPtr + m.y);
-        re = __ldg(a.rowPtr + m.y + 1);
+        if (m.y < a.nr) {  // (behind the last nonzero otherwise)
+            rs = __ldg(a.rowPtr + m.y);
+            re = __ldg(a.rowPtr + m.y + 1);
+        } else {
+            rs = m.x;
+        }
     }
     const bool here = m.x > rs && before.x <= rs;  // a row is cut here for the first time
     if (!here && !left) return;
+    const int base = a.based ? __ldg(a.rowPtr) : 0;
     const size_t col_step = cmb ? 1 : a.ldb, k_step = cmb ? a.ldb : 1;
     int kp = 1;
     while (kp < nv) kp <<= 1;
@@ -270,11 +282,11 @@ static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool c
         else if (a.beta != 1.0f || holds) *d = fmaf(a.beta, *d, x);
     };
     if (here) {
-        int last = min((re - 1) / a.chunk, a.nchunks - 1);  // the chunk of its last piece
+        const int last = min((re - 1 - base) / a.chunk, a.nchunks - 1);  // of its last piece
         const bool first_left = m.y - before.y > kStreamRows, last_left = many_rows(a, last);
         float x = 0.0f;
         if (k < nv) {
-            if (last_left) x = piece(x, last * a.chunk, re);
+            if (last_left) x = piece(x, base + last * a.chunk, re);
             if (first_left) x = piece(x, rs, m.x);
             for (long long q = c + sub; q <= last - last_left; q += subs)
                 x += __ldcg(a.slots + (q * 2) * nv + k);
@@ -303,7 +315,7 @@ static __global__ void __launch_bounds__(256) k_stream_fix(const KArgs a, bool c
         // last nonzero of the rows up to it.
 #pragma unroll
         for (int g = 0; g < T; ++g) {
-            const int h = min(max(p0[g] + max(len[g], 0) - 1, 0) / a.chunk, a.nchunks - 1);
+            const int h = min(max(p0[g] + max(len[g], 0) - 1 - base, 0) / a.chunk, a.nchunks - 1);
             m[g] = a.meta[h];
             next[g] = h + 1 < a.nchunks ? a.meta[h + 1].y : a.nr;
         }
@@ -384,8 +396,11 @@ inline void launch_stream_as(const KArgs &a, cudaStream_t st)
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, a.beta == 1.0f ? k_stream<NV, V, CMB, CMC, true>
-                                            : k_stream<NV, V, CMB, CMC, false>, a);
+    cudaLaunchKernelEx(&cfg,
+                       a.based          ? k_stream<NV, V, CMB, CMC, kStreamBased>
+                       : a.beta == 1.0f ? k_stream<NV, V, CMB, CMC, kStreamOne>
+                                        : k_stream<NV, V, CMB, CMC, kStreamPlain>,
+                       a);
     const int fix = stream_fix_ctas(a.nchunks, a.nr);
     if (fix > 0) {
         cfg.gridDim = dim3((unsigned)fix);

@@ -34,17 +34,18 @@ struct WinCols {
 
 // A piece of split row `row`, already stored in its carry slot by this worker,
 // arrives: piece_arrive for G lanes (`gmask`) and J vectors of V columns per
-// lane.  Templated on the kernel's types so that every kernel has its own
+// lane, in chunks counted from nonzero `base`.  Templated on the kernel's types so that every kernel has its own
 // copy: ptxas 12.9 crashes (at build time) on one copy shared by two kernels.
 template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK,
           int FORM>
 static __device__ __noinline__ void piece_arrive_win(const int *__restrict__ rowPtr, int *cnt,
                                                      const float *slots, float *C, int ldc,
                                                      int nv, int chunk, float beta, int row,
-                                                     int tb, int tiles, int tile, unsigned gmask)
+                                                     int tb, int tiles, int tile, unsigned gmask,
+                                                     int base)
 {
     const WinCols<G, V, J, MASK> cs{tb, nv};
-    const int rs = __ldg(rowPtr + row), re = __ldg(rowPtr + row + 1);
+    const int rs = __ldg(rowPtr + row) - base, re = __ldg(rowPtr + row + 1) - base;
     const int c0 = first_chunk(rs, chunk), c1 = last_chunk(re, chunk);
     __threadfence();
     __syncwarp(gmask);
@@ -389,14 +390,16 @@ __global__ void __launch_bounds__(256, MINB) k_win(const KArgs a)
                 tail = !cont;
             }
         }
+        // (a row is cut where chunks begin by count, so its chunk says where they are
+        // counted from: 0, or the first of a larger matrix's rows)
         if (head_piece)
             piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK, FORM>(
                 a.rowPtr, a.cnt, a.slots, a.C, a.ldc, a.nv, a.chunk, a.beta, r0, cs.tb, tiles, tile,
-                gmask);
+                gmask, k0 - c * a.chunk);
         if (tail)
             piece_arrive_win<G, V, J, U, TV, TB, MINB, BETA, MASK, FORM>(
                 a.rowPtr, a.cnt, a.slots, a.C, a.ldc, a.nv, a.chunk, a.beta, s1, cs.tb, tiles, tile,
-                gmask);
+                gmask, ke - (c + 1) * a.chunk);
         __syncwarp();
         // the next group from the tile's queue; a call makes exactly ngroups
         // claims, so a planned product counts on from where the last one ended

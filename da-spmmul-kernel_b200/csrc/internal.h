@@ -27,6 +27,7 @@ struct Resolved {
     int general;  // pipe 1, row-major: the masked window kernel's vector width (0: k_bal)
     int inner_chunk;  // pipe 5: the caller's chunk for the row-major product
     int l2_window;    // thousandths of B's lines marked L2-persisting (0 = off)
+    bool based;       // the row pointer may start anywhere, nnz be a larger matrix's
 };
 
 // SMs of the current device (148 when no device is visible).

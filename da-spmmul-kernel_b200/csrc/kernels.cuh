@@ -60,6 +60,7 @@ struct KArgs {
     int kahan_min;        // rows at least this long use compensated sums
     int l2_window;        // host side: thousandths of B's lines marked L2-persisting
     size_t b_bytes;       // host side: bytes of B (the window's extent)
+    int based;            // the nonzeros are [rowPtr[0], rowPtr[nr]), whatever nnz
 };
 
 // ---------------------------------------------------------------- vectors
@@ -553,6 +554,9 @@ __global__ void __launch_bounds__(256) k_fix_coo(const KArgs a)
 // The window kernel leaves rows without nonzeros to this pass: with C they are
 // finished here (C = beta*C, nv columns, the warp together; beta == 1 needs no pass
 // and gets no C, so such rows are not touched), with emap their bitmap is kept.
+// BASED: the rows are some of a larger matrix's, whose row pointer does not start at 0 and
+// whose nnz may be the matrix's (0.3 us more: a load that all wait for).
+template <bool BASED = false>
 static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowPtr,
                             int chunk, int snap, int nchunks, int2 *meta, int *cnt, int tiles,
                             unsigned int *head, unsigned int *emap, float *C, int nv, float beta)
@@ -563,9 +567,10 @@ static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowP
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const long long r0 = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
+    const int base = BASED ? __ldg(rowPtr) : 0, stop = BASED ? __ldg(rowPtr + nr) : nnz;
     if (r0 == 0) {
-        meta[0] = make_int2(0, 0);
-        meta[nchunks] = make_int2(nnz, nr);
+        meta[0] = make_int2(base, 0);
+        meta[nchunks] = make_int2(stop, nr);
         if (head)
             for (int t = 0; t < tiles; ++t) head[t] = 0;
     }
@@ -582,12 +587,15 @@ static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowP
                     dst[k] = beta == 0.0f ? 0.0f : fmaf(beta, dst[k], 0.0f);
             }
         }
+        if (BASED && r == nr - 1)  // boundaries behind the last nonzero
+            for (long long c = max(1LL, ((long long)re - base + chunk - 1) / chunk); c < nchunks; ++c)
+                meta[c] = make_int2(re, nr);
         if (rs == re) continue;
-        long long c = ((long long)rs + chunk - 1) / chunk;
+        long long c = ((long long)rs - base + chunk - 1) / chunk;
         if (c < 1) c = 1;
         bool split = false;
-        for (; c < nchunks && c * chunk < re; ++c) {
-            const int k = (int)(c * chunk);
+        for (; c < nchunks && base + c * chunk < re; ++c) {
+            const int k = (int)(base + c * chunk);
             const int kk = (k > rs && re - rs < snap) ? rs : k;
             meta[c] = make_int2(kk, (int)r);
             split |= kk > rs;
@@ -595,7 +603,7 @@ static __global__ void k_partition(int nr, int nnz, const int *__restrict__ rowP
         // a row split across chunks: its arrival counters (one per column
         // tile) live at its first chunk
         if (split && cnt)
-            for (int t = 0; t < tiles; ++t) cnt[(size_t)(rs / chunk) * tiles + t] = 0;
+            for (int t = 0; t < tiles; ++t) cnt[(size_t)((rs - base) / chunk) * tiles + t] = 0;
     }
 }
 
@@ -616,7 +624,8 @@ static __global__ void __launch_bounds__(256)
 }
 
 // Chunks holding pieces of a split row r (rows >= snap long are cut only at
-// nominal boundaries c*chunk, so the chunk of nonzero p inside r is p/chunk).
+// nominal boundaries c*chunk, so the chunk of nonzero p inside r is p/chunk; rs and re
+// are counted from the first row's start).
 __device__ __forceinline__ int first_chunk(int rs, int chunk) { return rs / chunk; }
 __device__ __forceinline__ int last_chunk(int re, int chunk) { return (re - 1) / chunk; }
 
