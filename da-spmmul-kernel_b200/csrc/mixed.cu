@@ -297,8 +297,10 @@ daspmm_status daspmm_spmm_mixed(const daspmm_config *cfg_in, int layout, int nr,
         const int L = cfg.lanes_col;  // the tile's width as resolve() has it
         const int W = L == 8 || L == 16 || L == 32 ? 4 * L
                                                    : (nv % 128 == 0 ? 128 : (nv % 64 == 0 ? 64 : 32));
-        cfg.chunk = window_chunk(nv, W, nr, nnz, nv == 128 ? 96 : 128);
-        if (!cfg.snap) cfg.snap = window_snap(cfg.chunk);
+        const int most = nv == 128 ? 96 : 128;
+        // (compensated rows are cut no more often than that: their pieces are added plainly)
+        cfg.chunk = kahan_min > 0 ? most : window_chunk(nv, W, nr, nnz, most);
+        if (!cfg.snap && kahan_min <= 0) cfg.snap = window_snap(cfg.chunk);
     }
     Resolved r;
     daspmm_status s = resolve(&cfg, layout, nr, nc, nnz, nv, nullptr, C, &r);
