@@ -459,9 +459,9 @@ static void launch_tma(const Resolved &r, const KArgs &a, cudaStream_t st)
     if (r.general) {
         launch_general(r, a, st);
     } else if (r.pipe == 4) {
-        if (r.W == 128) launch_lean<128, float, float, false>(r, a, st);
-        else if (r.W == 64) launch_lean<64, float, float, false>(r, a, st);
-        else launch_lean<32, float, float, false>(r, a, st);
+        if (r.W == 128) launch_win<128, float, float>(r, a, st);
+        else if (r.W == 64) launch_win<64, float, float>(r, a, st);
+        else launch_win<32, float, float>(r, a, st);
     } else if (r.pipe == 3) {
         launch_ring<1>(r, a, st);
     } else {

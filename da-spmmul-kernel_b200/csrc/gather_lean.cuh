@@ -1,8 +1,9 @@
-// gather_lean.cuh -- the balanced-CSR row-major SpMM kernels: k_win, the worker-
-// group window kernel that takes every product without compensated rows, and
-// k_bal_lean, the per-nonzero walk for products with Kahan rows.
+// gather_lean.cuh -- k_bal_lean, the per-nonzero walk of the balanced row-major
+// product for rows summed with Kahan compensation, and the loads, stores and element
+// conversions that it shares with the window kernel (gather_win.cuh), which takes every
+// other such product.
 //
-// Both take the chunks of the balanced split (k_partition).  A row split across
+// It takes the chunks of the balanced split (k_partition).  A row split across
 // chunks is finished inside the kernel: its last piece to arrive adds all
 // pieces in chunk order, so no fix-up launch is needed and a result does not
 // depend on scheduling.
@@ -11,8 +12,8 @@
 // TB in {float, bf16, fp16, fp8 e4m3}; products and sums are FP32.  For FP8
 // B, column k carries an FP32 scale (B = q * scale[k]); sums are taken over
 // the unscaled q and each output column is scaled once, when its row is
-// stored.  With KAHAN, rows of at least kahan_min nonzeros are summed with
-// Kahan compensation (each piece of a split row included).
+// stored.  Rows of at least kahan_min nonzeros are summed with Kahan compensation (each
+// piece of a split row included).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -144,7 +145,7 @@ __device__ __forceinline__ float ld_val(const T *p, uint64_t pol)
 // rows, beta != 0 and Kahan rows are all handled.  A row split across chunks
 // leaves its pieces in carry slots; the last piece to arrive adds them all
 // in chunk order (piece_arrive).  W / 32 elements of the B row per lane.
-template <int W, int U, typename TV, typename TB, bool KAHAN>
+template <int W, int U, typename TV, typename TB>
 __device__ __forceinline__ void lean_chunk(const KArgs &a, int c, int tile, int tiles,
                                            uint64_t pol_once)
 {
@@ -170,8 +171,8 @@ __device__ __forceinline__ void lean_chunk(const KArgs &a, int c, int tile, int 
 #pragma unroll
     for (int e = 0; e < VL; ++e) acc[e] = comp[e] = 0.0f;
     // Kahan rows: length of the current row (its start is the previous end)
-    int rs = KAHAN ? __ldg(a.rowPtr + r) : 0;
-    bool kh = KAHAN && re - rs >= a.kahan_min;
+    int rs = __ldg(a.rowPtr + r);
+    bool kh = re - rs >= a.kahan_min;
 
     const bool head_piece = cont;  // row m0.y continues from an earlier chunk
     auto emit = [&](int row, bool ends) {
@@ -204,11 +205,11 @@ __device__ __forceinline__ void lean_chunk(const KArgs &a, int c, int tile, int 
                 rc = rn;
                 rn = __ldg(a.rowPtr + min(rb + 33 + lane, a.nr));
             }
-            if constexpr (KAHAN) rs = re;
+            rs = re;
             re = __shfl_sync(kFull, rc, r - rb);
-            if constexpr (KAHAN) kh = re - rs >= a.kahan_min;
+            kh = re - rs >= a.kahan_min;
         }
-        if (KAHAN && kh) {
+        if (kh) {
 #pragma unroll
             for (int e = 0; e < VL; ++e) {  // Kahan: carry the rounding error along
                 const float y = fmaf(v, b[e], -comp[e]);
@@ -273,7 +274,7 @@ __device__ __forceinline__ void lean_chunk(const KArgs &a, int c, int tile, int 
     if (tail_piece) piece_arrive<VL>(a, s1, tb, tiles, tile);
 }
 
-template <int W, int U, typename TV = float, typename TB = float, bool KAHAN = false>
+template <int W, int U, typename TV, typename TB>
 __global__ void __launch_bounds__(256, DASPMM_LEAN_MINB) k_bal_lean(const KArgs a)
 {
     const int lane = threadIdx.x & 31;
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(256, DASPMM_LEAN_MINB) k_bal_lean(const KArgs 
     // and no wave of chunks is left half-used.
     long long cl = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     while (cl < a.nchunks) {
-        lean_chunk<W, U, TV, TB, KAHAN>(a, (int)cl, blockIdx.y, gridDim.y, pol_once);
+        lean_chunk<W, U, TV, TB>(a, (int)cl, blockIdx.y, gridDim.y, pol_once);
         unsigned int nx = 0;
         if (lane == 0) nx = atomicAdd(a.head + blockIdx.y, 1u);
         cl = nwarps + (long long)__shfl_sync(kFull, nx, 0);

@@ -10,8 +10,9 @@
 // Rows without nonzeros fall out of the row loop; a chunk with more than kStreamRows rows
 // is left to k_stream_fix, whose warps share out the rows (a million rows of 8, the lower
 // half empty, N = 1 / 8 670 / 2043 us when one CTA walked them, 37 / 65 so; column-major
-// N = 8 6027 and 128).  A chunk's boundary moves down to the start of a row shorter than kStreamSnap; longer rows are cut there, each
-// piece leaves its sum in a slot and k_stream_fix adds the slots in chunk order.
+// N = 8 6027 and 128).  A chunk's boundary moves down to the start of a row shorter than
+// kStreamSnap; longer rows are cut there, each piece leaves its sum in a slot and
+// k_stream_fix adds the slots in chunk order.
 // No partition pass: two warps of the CTA find the chunk's rows by a 32-way search
 // while the others load (so the chunk's load starts kStreamSnap - 1 nonzeros
 // early, where its boundary can be).
@@ -27,15 +28,16 @@
 
 namespace daspmm {
 
-// Up to here k_stream, above the window kernel: at 8 / 12 / 16 columns 29 / 47 / 40 us
-// against 33 / 39 / 37 on the 262k power-law matrix, 33 / 47 / 51 against 33 / 34 / 34 on
-// a uniform-random one (at 4 columns 24 and 31; the gather before both took 82 and
-// 39 at 4, 97 and 54 at 8, 106 and 82 at 16).
+// Up to here k_stream, above the window kernel.  us of either on the 262k power-law
+// matrix / a uniform-random one of 8 per row when the line was drawn: 8 columns 29 / 33
+// and 33 / 33, 12 columns 47 / 47 and 39 / 34, 16 columns 40 / 51 and 37 / 34 (k_stream at 8 now
+// 26 / 26; the gather before both 97 / 54 at 8, 106 / 82 at 16).
 constexpr int kStreamMaxNv = 8;
 constexpr int kStreamSnap = 64;
 constexpr int kStreamLong = 96;  // nonzeros from which on a warp sums a row
 constexpr int kStreamPlain = 0, kStreamOne = 1, kStreamBased = 2;  // see k_stream
-constexpr int kStreamRows = 4096;  // a chunk of more rows is left to k_stream_fix
+constexpr int kStreamRows = 4096;  // a chunk of more rows is left to k_stream_fix (a CTA
+                                   // walks so many in 16 turns at one column)
 
 // Shared memory of a chunk: values, and the rows of B (see pitch in k_stream).
 inline size_t stream_smem(int chunk, int nv, bool cmc)

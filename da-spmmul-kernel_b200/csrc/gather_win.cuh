@@ -20,7 +20,7 @@ __device__ __forceinline__ void ld_bytes(uint32_t (&w)[NB >= 4 ? NB / 4 : 1], co
 }
 
 // Two choices that give the same bits and differ in what the compiler makes of the
-// window loop; each shape has the faster one (launch_win).
+// window loop; each shape has the one that measures best (see launch_win).
 constexpr int kFormLate = 1;  // a nonzero's value is fetched from its lane with its sum, not
                               // with its load
 constexpr int kFormLim = 2;   // a window's end is kept, not its length
@@ -481,11 +481,28 @@ inline bool win_aligned(const KArgs &a, int V)
 //   BF16 values, E4M3 B: 36.5 / 46.4 / 65.4 / 130 [45.1 / 45.4 / 64.6 / 131], random
 //     41.2 / 51.6 / 81.9 / 143 [51.5 / 65.9 / 98.4 / 181]
 // FP32 rows of 128 columns take 16-lane workers with 32-byte loads; 2-byte B 16
-// rows in flight (their registers are those of 8 FP32 rows); the narrower tiles
+// rows in flight (their registers are those of 8 FP32 rows; a worker's lanes are the
+// most: 8 rows with 8 lanes); the narrower tiles
 // of 2- and 1-byte B 8-byte loads in 24 warps per SM, E4M3 in 32 columns 4-byte
 // ones (8-lane workers: windows of 8 nonzeros, against 4 with 8-byte loads,
 // 54.7 and 46.0 us); E4M3 in 128 columns 8-byte loads in 16-lane workers for one
 // tile, 16-byte loads in 8-lane ones for wider products.
+// The loop's form (kFormLate, kFormLim), us on the power-law matrix / the uniform-random one
+// with none, late, lim, both; what is taken stands first:
+//   FP32     N = 32 none 34.6 / 39.4, 36.0 / 42.7, 34.9 / 39.9, 38.1 / 48.1; N = 64 none 56 / 57,
+//            58 / 59, 63 / 66, 58 / 59; N = 128 none 84.6 / 121, 92 / 132, 83.9 / 121, 85.7 / 123
+//   BF16     N = 32 late 36.3 / 39.3, none 36.9 / 39.1, lim 35.9 / 38.5, both 36.3 / 39.6; N = 64
+//            none 45.1 / 49.7, 46.1 / 52.0, 46.3 / 52.3, 46.4 / 53.1; N = 128 both 66.6 / 84.7,
+//            none 69.9 / 87.9, late 68.4 / 85.7, lim 68.3 / 85.6
+//   FP16     N = 32 none 34.8 / 37.5, 37.1 / 43.1, 34.7 / 37.3, 35.4 / 39.8; N = 64 lim 43.5 /
+//            47.9, none 45.0 / 50.8, late 45.3 / 50.9, both 45.6 / 52.6; N = 128 both 64.4 / 80.0,
+//            none 70.3 / 89.3, late 69.6 / 87.7, lim 65.7 / 80.8 (uniform rows of 20 lose: 73.6,
+//            lim 71.4)
+//   E4M3 B   N = 32 both 35.8 / 37.6, none 36.0 / 38.5, late 36.6 / 41.6, lim 36.0 / 38.4; N = 64
+//            none 46.3 / 50.3, 46.8 / 52.7, 47.8 / 54.2, 46.2 / 52.0; N = 128 lim 61.3 / 72.1, none
+//            61.9 / 73.0, late 63.1 / 75.6, both 62.5 / 74.2; N = 256 late 128.5 / 142.6, none 133 /
+//            151, lim 133 / 150, both 128.9 / 143.5
+//   masked   none: N = 41 57.5 / 59.1, 58.9 / 61.3, 57.2 / 59.2, 59.0 / 61.7
 template <int W, typename TV, typename TB>
 inline void launch_win(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
@@ -509,30 +526,25 @@ inline void launch_win(const Resolved &r, const KArgs &a, cudaStream_t st)
     } else if constexpr (W == 64) {
         constexpr int V = b2 ? 4 : 8;
         if (win_aligned<TB>(a, V))
-            return launch_win_as<64 / V, V, 1, f32 ? 8 : 16, TV, TB, f32 ? 2 : 3, false,
+            return launch_win_as<64 / V, V, 1, 64 / V, TV, TB, f32 ? 2 : 3, false,
                                  f16 ? kFormLim : 0>(r, a, st);
         launch_win_as<16, 2, 2, 8, TV, TB, 3, false>(r, a, st);
     } else {
         if (win_aligned<TB>(a, 4))
-            return launch_win_as<8, 4, 1, b2 ? 16 : 8, TV, TB, 3, false,
+            return launch_win_as<8, 4, 1, 8, TV, TB, 3, false,
                                  f32 || f16 ? 0 : b2 ? kFormLate : kFormLate | kFormLim>(r, a, st);
         launch_win_as<16, 1, 2, 8, TV, TB, 3, false>(r, a, st);
     }
 }
 
-// The balanced product of one column-tile width: the window kernel, or the
-// walk for products with Kahan rows.
-template <int W, typename TV, typename TB, bool K>
-inline void launch_lean(const Resolved &r, const KArgs &a, cudaStream_t st)
+// The walk for products with Kahan rows.
+template <int W, typename TV, typename TB>
+inline void launch_walk(const Resolved &r, const KArgs &a, cudaStream_t st)
 {
-    if constexpr (K) {
-        const unsigned gx = (unsigned)std::max<long long>(
-            1, std::min<long long>(((long long)a.nchunks + 7) / 8,
-                                   (long long)device_sms() * DASPMM_LEAN_MINB));
-        launch_pdl(k_bal_lean<W, DASPMM_LEAN_U, TV, TB, true>, dim3(gx, r.tiles), st, a);
-    } else {
-        launch_win<W, TV, TB>(r, a, st);
-    }
+    const unsigned gx = (unsigned)std::max<long long>(
+        1, std::min<long long>(((long long)a.nchunks + 7) / 8,
+                               (long long)device_sms() * DASPMM_LEAN_MINB));
+    launch_pdl(k_bal_lean<W, DASPMM_LEAN_U, TV, TB>, dim3(gx, r.tiles), st, a);
 }
 
 }  // namespace daspmm

@@ -12,19 +12,13 @@
 
 namespace daspmm {
 
-template <int W, typename TV, typename TB, bool K>
-static void launch_mixed_w(const Resolved &r, const KArgs &a, cudaStream_t st)
-{
-    launch_lean<W, TV, TB, K>(r, a, st);
-}
-
 template <typename TV, typename TB>
 static void launch_mixed(const Resolved &r, const KArgs &a, bool kahan, cudaStream_t st)
 {
 #define DASPMM_MW(w)                                                                        \
     if (r.W == w) {                                                                         \
-        if (kahan) launch_mixed_w<w, TV, TB, true>(r, a, st);                               \
-        else launch_mixed_w<w, TV, TB, false>(r, a, st);                                   \
+        if (kahan) launch_walk<w, TV, TB>(r, a, st);                                        \
+        else launch_win<w, TV, TB>(r, a, st);                                               \
         return;                                                                             \
     }
     DASPMM_MW(128) DASPMM_MW(64) DASPMM_MW(32)

@@ -74,8 +74,9 @@ extern "C" daspmm_status daspmm_spmm_noalloc(int layout, int nr, int nc, int nnz
     void *scratch = nullptr;
     s = scratch_address(&scratch);
     if (s != DASPMM_OK) return s;
-    // Every scratch entry the kernels read (boundary table, carry slots) is
-    // written earlier in the same call, so nothing needs clearing between calls.
+    // Every scratch entry the kernels read (boundary table, carry slots) is written
+    // earlier in the same call, but for the word that tells k_stream_fix whether rows were
+    // left, which may hold anything: nothing needs clearing between calls.
     return daspmm::run_resolved(r, layout, nr, nc, nnz, nv, rowPtr, nullptr, colIdx, values, B,
                                 C, beta, scratch, (size_t)DASPMM_NOALLOC_MAX_BYTES,
                                 (cudaStream_t)stream);

@@ -124,7 +124,7 @@ std::vector<daspmm_config> candidates(int layout, int nv, bool have_coo)
     }
     if (layout == DASPMM_ROW_MAJOR && nv % 32 == 0) {
         // the window kernel: chunk sizes at the widest tile, then narrower
-        // column tiles (64 / 32 floats: G = 8 / the 32-lane kernel)
+        // column tiles (64 and 32 floats)
         for (int ch : {64, 96, 128, 256}) add(DASPMM_ALG_CSR_BALANCED, 4, ch);
         for (int L : {16, 8})
             if (nv % (4 * L) == 0 && (nv % 128 == 0 || (L == 8 && nv % 64 == 0)))
