@@ -1036,6 +1036,7 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
     Resolved r;
     c.alg = alg == DASPMM_ALG_AUTO ? DASPMM_ALG_CSR_SCALAR : alg;
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
+    const size_t own_need = workspace_bytes(r, nv);
     c.alg = DASPMM_ALG_CSR_BALANCED;
     if (resolve(&c, layout, nr, nc, nnz, nv, B, C, &r) != DASPMM_OK) return DASPMM_OK;
     const size_t rows = coo ? align256(sizeof(int) * ((size_t)nr + 1)) : 0;
@@ -1044,6 +1045,13 @@ static daspmm_status through_balanced(int alg, int layout, int nr, int nc, int n
     void *ws = scratch.take(rows + need);
     if (!ws) return DASPMM_OK;
     char *own = (char *)ws + rows;
+    if (own_need) {
+        // The same call inside a capture runs its own kernel, which needs the stream's
+        // workspace: a call before it must have made that, as it does for the others.
+        const WorkspaceLock hold = hold_workspace(st);
+        void *block = nullptr;
+        if (cached_workspace(own_need, st, &block) != DASPMM_OK) cudaGetLastError();
+    }
     if (coo) {
         // where the row-major product's boundaries will lie (k_stream keeps none)
         Resolved in = r;

@@ -103,6 +103,28 @@ def test_while_another_stream_is_captured(mat, alg, layout, nv):
     _check(A, layout, nv, B2, C2)
 
 
+@pytest.mark.parametrize("alg", [D.Alg.COO_SCALAR, D.Alg.COO_VECTOR])
+@pytest.mark.parametrize("layout,nv", [(0, 4), (0, 64), (1, 32)])
+def test_captured_after_the_same_call(mat, alg, layout, nv):
+    """The call before a capture leaves what the captured one needs (COO's own kernels
+    have a workspace), though it ran as the balanced product itself."""
+    import torch
+    A, dA = mat
+    st = torch.cuda.Stream()
+    B, Bt, C = _operands(A, nv)
+    D.spmm(alg, layout, dA, Bt, C, beta=1.0, nv=nv, stream=st)
+    torch.cuda.synchronize()
+    _check(A, layout, nv, B, C)
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=st):
+        D.spmm(alg, layout, dA, Bt, C, beta=1.0, nv=nv, stream=st)
+    C.zero_()
+    torch.cuda.synchronize()
+    g.replay()
+    torch.cuda.synchronize()
+    _check(A, layout, nv, B, C)
+
+
 def test_memory_is_given_back(mat):
     import torch
     A, dA = mat
