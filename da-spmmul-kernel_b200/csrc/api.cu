@@ -520,7 +520,8 @@ static daspmm_status dispatch(const Resolved &r, KArgs &a, dim3 grid, dim3 fix_g
     return DASPMM_ERR_UNSUPPORTED;
 }
 
-// dst (Cn x R, row-major) = transpose of src (R x Cn, row-major) + beta * dst.  KEEP: the columns of dst whose row of the matrix is empty are left as they are.
+// dst (Cn x R, row-major) = transpose of src (R x Cn, row-major) + beta * dst.  KEEP: the
+// columns of dst whose row of the matrix is empty are left as they are.
 template <int TR, bool KEEP>
 static void launch_transpose_tr(const float *src, long long R, long long Cn, float *dst,
                                 float beta, const int *rowPtr, cudaStream_t st)
@@ -780,9 +781,10 @@ void launch_partition(const Resolved &r, int nr, int nnz, const int *rowPtr, con
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, r.based ? k_partition<true> : k_partition<false>, nr, nnz, rowPtr, (int)r.chunk, (int)r.snap,
-                       (int)r.nchunks, const_cast<int2 *>(a.meta), a.cnt, (int)r.tiles, a.head,
-                       a.emap, rows_beta && a.beta != 1.0f ? a.C : (float *)nullptr, a.nv, a.beta);
+    cudaLaunchKernelEx(&cfg, r.based ? k_partition<true> : k_partition<false>, nr, nnz, rowPtr,
+                       (int)r.chunk, (int)r.snap, (int)r.nchunks, const_cast<int2 *>(a.meta), a.cnt,
+                       (int)r.tiles, a.head, a.emap,
+                       rows_beta && a.beta != 1.0f ? a.C : (float *)nullptr, a.nv, a.beta);
     count_launches(1);
 }
 

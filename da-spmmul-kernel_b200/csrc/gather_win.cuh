@@ -34,8 +34,9 @@ struct WinCols {
 
 // A piece of split row `row`, already stored in its carry slot by this worker,
 // arrives: piece_arrive for G lanes (`gmask`) and J vectors of V columns per
-// lane, in chunks counted from nonzero `base`.  Templated on the kernel's types so that every kernel has its own
-// copy: ptxas 12.9 crashes (at build time) on one copy shared by two kernels.
+// lane, in chunks counted from nonzero `base`.  Templated on the kernel's types so that
+// every kernel has its own copy: ptxas 12.9 crashes (at build time) on one copy shared by
+// two kernels.
 template <int G, int V, int J, int U, typename TV, typename TB, int MINB, bool BETA, bool MASK,
           int FORM>
 static __device__ __noinline__ void piece_arrive_win(const int *__restrict__ rowPtr, int *cnt,

@@ -5,7 +5,7 @@
  *
  * TEST INFRASTRUCTURE ONLY.  Only tests/, __graft_entry__.smoke() and the
  * cpu_baseline and reference legs of bench.py may load this library, and only
- * as the checker (or, in the reference leg, to build that leg's inputs).
+ * as the oracle (or, in the reference leg, to build that leg's inputs).
  * The shipped library (libdaspmm.so) never links or calls it.
  *
  * Every function cites the reference file:line it restates (paths relative to

@@ -2,7 +2,7 @@
 harness around the unmodified reference (_ref/libref.so).
 
 TEST INFRASTRUCTURE ONLY: imported by tests/, __graft_entry__.smoke() and the
-cpu_baseline / reference legs of bench.py, as the checker.  The product
+cpu_baseline / reference legs of bench.py, as the oracle.  The product
 (libdaspmm.so and its bindings) never imports this module.
 
 Each function names the reference code it restates (see oracle.c).
